@@ -45,3 +45,28 @@ def test_open_list_overflow_is_reported(gpu_lib):
     with G.AStarRef(64, 64, slots=1, open_capacity=16) as a:
         r = a.solve(m, agents)
     assert r[0]["status"] == 3  # GPQ_ERR_QUEUE_FULL
+
+
+@pytest.mark.parametrize("w,h,frac", [(1, 300, 0.0), (300, 1, 0.0), (9, 8, 0.1), (200, 200, 0.0), (2048, 2048, 0.2),
+                                      (8192, 512, 0.2), (8193, 9, 0.1), (2049, 2048, 0.2)])
+def test_vertex_forms(gpu_lib, w, h, frac):
+    """Sizes at the edges of the packed vertex word (up to 22 coordinate bits, sides up to
+    8,192; beyond them the general form) and open lists of one to thousands of vertices:
+    agents between nearby cells all over the map, one that starts on its goal, and -- on the
+    small maps -- one whose goal is walled in, so that the whole map is searched."""
+    m = G.astar_ref_map(w, h, frac, 1.0, seed=w + h) if frac else np.zeros((h, w), np.uint8)
+    rng = np.random.default_rng(w * 7 + h)
+    free = lambda x, y: m[y, x] == 0  # noqa: E731
+    pairs = []
+    while len(pairs) < 40:
+        x0, y0 = int(rng.integers(w)), int(rng.integers(h))
+        x1, y1 = (int(np.clip(v + rng.integers(-40, 41), 0, n - 1)) for v, n in ((x0, w), (y0, h)))
+        if free(x0, y0) and free(x1, y1):
+            pairs.append((y0 * w + x0, y1 * w + x1))
+    pairs.append((pairs[0][0], pairs[0][0]))
+    if w == 200:
+        gx, gy = 150, 40
+        m[gy - 1:gy + 2, gx - 1:gx + 2] = 1
+        m[gy, gx] = 0
+        pairs.append((120 * w + 17, gy * w + gx))
+    _check(m, np.array(pairs, G.ASTAR_REF_AGENT_DTYPE), slots=7)
