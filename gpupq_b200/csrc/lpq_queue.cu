@@ -59,15 +59,16 @@ __global__ void lpq_post_kernel(LpqDev q, gpq_item* ibuf, uint32_t* icnt, uint32
       }
     } else {
       const LsqView v{q.items + base, q.links + base};
-      uint32_t root = q.root[lp], ftop = q.freetop[lp];
+      LsqRoot root = lsq_load_root(v, q.root[lp]);
+      uint32_t ftop = q.freetop[lp];
       for (uint32_t j = 0; j < k; ++j) {
         if (ftop == 0) { gpq_set_error(&ctr->err, GPQ_ERR_QUEUE_FULL); break; }
         const uint32_t x = q.freestk[base + --ftop];
         v.it[x] = src[j];
-        root = lsq_insert(v, root, x);
+        root = lsq_insert(v, root, x, v.key(x));
         ++n;
       }
-      q.root[lp] = root;
+      q.root[lp] = root.t;
       q.freetop[lp] = ftop;
     }
     q.size[lp] = n;
@@ -83,7 +84,8 @@ __device__ __forceinline__ bool lpq_peek(const LpqDev& q, uint32_t lp, gpq_item*
     return true;
   }
   const LsqView v{q.items + base, q.links + base};
-  const uint32_t r = lsq_splay(v, q.root[lp], 0ull);
+  uint64_t rm;
+  const uint32_t r = lsq_splay(v, lsq_load_root(v, q.root[lp]), 0ull, &rm).t;
   q.root[lp] = r;
   *out = v.it[r];
   return true;
@@ -118,19 +120,21 @@ __global__ void lpq_pop_kernel(LpqDev q, uint32_t L, float bound, uint32_t max_p
       }
     } else {
       const LsqView v{q.items + base, q.links + base};
-      uint32_t root = q.root[lp], ftop = q.freetop[lp];
-      while (root != kLsqNil && (max_per_lp == 0 || c < max_per_lp)) {
-        root = lsq_splay(v, root, 0ull);
-        const gpq_item e = v.it[root];
+      LsqRoot root = lsq_load_root(v, q.root[lp]);
+      uint32_t ftop = q.freetop[lp];
+      while (root.t != kLsqNil && (max_per_lp == 0 || c < max_per_lp)) {
+        uint64_t rm;
+        root = lsq_splay(v, root, 0ull, &rm);
+        const gpq_item e = v.it[root.t];
         if (!(e.ts < bound)) break;
         tmp[base + c++] = e;
-        const uint32_t x = root;
-        root = v.right(x);
+        const uint32_t x = root.t;
+        root = lsq_load_root(v, root.ln & 0xffffu);
         v.it[x].lp = 0xffffffffu;
         q.freestk[base + ftop++] = (uint16_t)x;
         --n;
       }
-      q.root[lp] = root;
+      q.root[lp] = root.t;
       q.freetop[lp] = ftop;
     }
     q.size[lp] = n;

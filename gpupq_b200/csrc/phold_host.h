@@ -82,8 +82,20 @@ inline gpq_status lab_geometry(const gpq_phold_config& c, LabGeometry* g) {
   return GPQ_OK;
 }
 
+// Lanes per LP of the splay queue: one lane works on a tree, and lanes of a warp on
+// different trees take different paths, so they run one after another: an LP gets as wide
+// a group as one wave of threads (148 SMs x 1,024) allows.  Measured (16 events per LP,
+// lookahead 1, end time 100; ms a run with 1 / 4 / 16 / 32 lanes): 1,024 LPs 13.0 / 4.9 /
+// 3.2 / 2.4, 8,191 LPs 14.1 / 5.3 / 5.2 / 6.6; 36,473 LPs to end time 50 7.2 / 4.6 / 8.8 /
+// 9.2; 65,536 LPs to end time 30 4.8 / 5.8 (1 / 4 lanes).
+inline uint32_t lsq_lanes(uint32_t num_lps) {
+  for (uint32_t g = 32; g >= 4; g >>= 1)
+    if ((uint64_t)num_lps * g <= 148u * 1024u) return g;
+  return 1;
+}
+
 // Fills the per-kind defaults (capacity 256, insert capacity 64, 256-thread CTAs,
-// 8 lanes per LP; one lane for the splay queue) and checks them.
+// 8 lanes per LP; lsq_lanes for the splay queue) and checks them.
 inline gpq_status normalize_queue_config(gpq_phold_config* c) {
   if (c->capacity == 0) c->capacity = 256;
   if (c->insert_capacity == 0) c->insert_capacity = 64;
@@ -97,7 +109,7 @@ inline gpq_status normalize_queue_config(gpq_phold_config* c) {
   if (c->block_threads == 0) c->block_threads = 256;
   GPQ_CHECK_ARG(c->block_threads % 32 == 0 && c->block_threads >= 32 && c->block_threads <= 1024,
                 "block_threads must be a multiple of 32 in [32, 1024]");
-  if (c->queue_kind == GPQ_QUEUE_LSQ) c->lanes_per_lp = 1;
+  if (c->queue_kind == GPQ_QUEUE_LSQ) c->lanes_per_lp = lsq_lanes(c->num_lps);
   if (c->lanes_per_lp == 0) c->lanes_per_lp = 8;
   if (c->queue_kind == GPQ_QUEUE_LAQ)
     GPQ_CHECK_ARG(c->lanes_per_lp == 4 || c->lanes_per_lp == 8 || c->lanes_per_lp == 16 || c->lanes_per_lp == 32,

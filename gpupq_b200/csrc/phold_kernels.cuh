@@ -34,7 +34,8 @@ template <int G>
 struct LhqP : LhqPolicy<G> {
   __device__ static LhqDev dev(const LpQueueDev& l) { return LhqDev{l.items, l.a, l.cap_log2}; }
 };
-struct LsqP : LsqPolicy {
+template <int G>
+struct LsqP : LsqPolicy<G> {
   __device__ static LsqDev dev(const LpQueueDev& l) {
     return LsqDev{l.items, l.links, l.freestk, l.a, l.b, l.c, l.cap_log2};
   }
@@ -284,7 +285,13 @@ inline bool phold_kernel_set(uint32_t kind, uint32_t group, uint32_t ibc, PholdK
       case 32: GPQ_KS(LhqP<32>);
     }
   } else if (kind == GPQ_QUEUE_LSQ) {
-    GPQ_KS(LsqP);
+    switch (group) {
+      case 1: GPQ_KS(LsqP<1>);
+      case 4: GPQ_KS(LsqP<4>);
+      case 8: GPQ_KS(LsqP<8>);
+      case 16: GPQ_KS(LsqP<16>);
+      case 32: GPQ_KS(LsqP<32>);
+    }
   }
 #undef GPQ_KS
   return false;
