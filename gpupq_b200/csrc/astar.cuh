@@ -139,26 +139,63 @@ __device__ __forceinline__ void astar_inbox_push(const AstarDev& d, AstarInstDev
 // global copy with atomicMin (a filter for their sends) and the holder merges its copy
 // back with atomicMin when it lets go of the tile.
 struct AstarTileSmem {
-  uint2* fa;      // frontier buffers [frontier_cap]
-  uint2* fb;
+  uint2* fa;      // items to expand at the start of the visit; frontier buffer [frontier_cap]
+  uint2* fb;      // list walk: second frontier buffer
   uint32_t* gt;   // [ts * ts] g of the tile's cells, local index ly * ts + lx
   uint32_t* blk;  // [ts * ts / 32] blocked bits of the tile
-  uint32_t* chg;  // [ts * ts / 32] cells whose g dropped during this visit
-  uint2* ob;      // [8 * ts] moves into other tiles, sent when the visit ends
+  uint32_t* chg;  // list walk: [ts * ts / 32] cells whose g dropped during this visit
+  uint2* ob;      // list walk: [8 * ts] moves into other tiles, sent when the visit ends
+  uint16_t* vs;   // sweeps: [ts + 2][astar_sweep_stride] g - g_min of the expanded cells
+  uint32_t flag[2][10];  // sweeps: warps whose cells changed, by parity, a zero at each end
   uint32_t ob_n;
   uint32_t n[3];  // frontier fill, rotating by level
   uint32_t ub;    // the instance's best goal cost as of this visit (stale values only prune less)
   uint32_t open_min;
   uint32_t open_cnt;
+  uint32_t g_min;  // of the items to expand
   unsigned long long pops;
   uint32_t scan[33];
 };
 
 __host__ __device__ inline uint32_t astar_outbox_cap(uint32_t ts) { return 8u * ts; }
 
-__host__ __device__ inline size_t astar_smem_bytes(uint32_t ts, uint32_t frontier_cap) {
+// How a visit walks its tile: a CTA with a thread for 16 cells sweeps tiles of 64 x 64 and
+// 32 x 32 cells (astar_sweep_tile); other tile sides, smaller CTAs, and tiles worked by one
+// warp keep frontier lists (astar_expand_warp).
+__host__ __device__ inline bool astar_sweeps(uint32_t ts, bool warp, uint32_t block) {
+  return !warp && (ts == 64u || ts == 32u) && block >= ts * ts / 16u;
+}
+
+// 16-bit cells of a row in shared memory: 8 in front of the tile's (a 16-byte border, of which
+// the last is the left neighbour), 16 or more behind; rows shift by 12 banks (tiles of 64)
+// so that eight lanes' 16-byte loads from two rows meet 32 different banks.
+__host__ __device__ inline uint32_t astar_sweep_stride(uint32_t ts) { return ts + 24u; }
+
+__host__ __device__ inline size_t astar_smem_bytes(uint32_t ts, uint32_t frontier_cap, bool warp, uint32_t block) {
+  const size_t cells = (size_t)ts * ts, words = cells / 32;
+  if (astar_sweeps(ts, warp, block))
+    return (size_t)(ts + 2u) * astar_sweep_stride(ts) * sizeof(uint16_t) + (size_t)frontier_cap * sizeof(uint2) +
+           cells * sizeof(uint32_t) + words * sizeof(uint32_t);
   return 2ull * frontier_cap * sizeof(uint2) + (size_t)astar_outbox_cap(ts) * sizeof(uint2) +
-         (size_t)ts * ts * sizeof(uint32_t) + 2ull * (ts * ts / 32) * sizeof(uint32_t);
+         cells * sizeof(uint32_t) + 2ull * words * sizeof(uint32_t);
+}
+
+__device__ __forceinline__ void astar_smem_carve(AstarTileSmem& sm, unsigned char* base, uint32_t ts,
+                                                 uint32_t frontier_cap, bool warp) {
+  const uint32_t words = ts * ts / 32;
+  if (astar_sweeps(ts, warp, blockDim.x)) {
+    sm.vs = reinterpret_cast<uint16_t*>(base);
+    sm.gt = reinterpret_cast<uint32_t*>(sm.vs + (ts + 2u) * astar_sweep_stride(ts));
+    sm.fa = reinterpret_cast<uint2*>(sm.gt + ts * ts);
+    sm.blk = reinterpret_cast<uint32_t*>(sm.fa + frontier_cap);
+    return;
+  }
+  sm.fa = reinterpret_cast<uint2*>(base);
+  sm.fb = sm.fa + frontier_cap;
+  sm.ob = sm.fb + frontier_cap;
+  sm.gt = reinterpret_cast<uint32_t*>(sm.ob + astar_outbox_cap(ts));
+  sm.blk = sm.gt + ts * ts;
+  sm.chg = sm.blk + words;
 }
 
 // Geometry of the tile being processed.
@@ -379,6 +416,252 @@ __device__ __forceinline__ uint32_t astar_worker_scan(uint32_t flag, uint32_t* s
   return astar_block_scan(flag, scratch, total);
 }
 
+// ---- sweeps ----
+//
+// The labels of a visit come from relaxing the whole tile until nothing changes: a thread
+// holds 16 cells of a row as 15-bit labels (g - g_min of the visit's items), two to a
+// register, and one sweep takes the minimum over a cell's neighbours with the packed
+// add-minimum instructions.  A search is a chain of visits -- a round waits for its slowest
+// tile -- and a visit's time is its number of steps times the latency of one: a sweep moves
+// every wavefront of the tile by one cell in about 250 cycles without lists, atomics or
+// per-cell branches, where a level of a frontier list costs a pass through shared-memory
+// counters and appends.  Warps whose rows and neighbour rows did not change skip a sweep.
+// Measured, search only: 2048 x 2048 4-connected 8.05 -> 2.45 ms, 500 8-connected searches
+// of sides 64 to 1,024 12.0 -> 3.7 ms.
+//
+// Only cells that this visit labels, and its items, pass their label on, and only inside
+// the window (label < K): the others' moves were made when they were labelled.  Labels only
+// fall, so a sweep may read a neighbour's label before or after its update.
+
+static constexpr uint32_t kSweepInf = 0x7fffu;        // no label
+static constexpr uint32_t kSweepInf2 = 0x7fff7fffu;
+static constexpr uint32_t kSweepSpan = 0x7f00u;       // larger labels are not passed on in this visit
+// Sweeps of a warp between barriers (fewer when its cells stop changing): the 2048 x 2048
+// search takes 3.69 / 3.07 / 2.64 / 2.45 ms with 1 / 2 / 4 / 8.
+static constexpr uint32_t kSweepsPerBarrier = 8;
+static constexpr uint32_t kSweepMax = 1u << 16;       // sweeps of one visit (at most one per cell is needed)
+
+__device__ __forceinline__ uint32_t astar_pair_perm(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
+}
+
+// The labels v below k, the others as "no label" (both halves; k as (k | 0x8000) - 1).
+__device__ __forceinline__ uint32_t astar_pair_below(uint32_t v, uint32_t k1) {
+  const uint32_t ok = astar_pair_perm(k1 - v, 0u, 0xbb99u);  // the halves' top bits, spread: v < k
+  return v | (~ok & kSweepInf2);
+}
+
+// Pairs shifted by one cell along a row of eight pairs p with neighbours a (left) and b (right).
+__device__ __forceinline__ uint32_t astar_pair_left(const uint32_t* p, int i, uint32_t a) {
+  return astar_pair_perm(i ? p[i ? i - 1 : 0] : a, p[i], 0x5432u);
+}
+__device__ __forceinline__ uint32_t astar_pair_right(const uint32_t* p, int i, uint32_t b) {
+  return astar_pair_perm(p[i], i < 7 ? p[i < 7 ? i + 1 : 7] : b, 0x5432u);
+}
+
+__device__ __forceinline__ void astar_load_row(const uint16_t* row, uint32_t* p, uint32_t& a, uint32_t& b) {
+  const uint4 u = *reinterpret_cast<const uint4*>(row), v = *reinterpret_cast<const uint4*>(row + 8);
+  p[0] = u.x; p[1] = u.y; p[2] = u.z; p[3] = u.w;
+  p[4] = v.x; p[5] = v.y; p[6] = v.z; p[7] = v.w;
+  a = *reinterpret_cast<const uint32_t*>(row - 2);
+  b = *reinterpret_cast<const uint32_t*>(row + 16);
+}
+
+// Walks the tile from the n items of sm.fa (all threads; sm.g_min is set, sm.vs all "no
+// label").  On return sm.vs holds the labels of the expanded cells; changed labels are
+// merged into the global g values, labelled cells above the window are in the open array.
+// DIAG: 8-connected, costs 10 and 14; else unit moves.
+template <bool DIAG>
+__device__ __forceinline__ void astar_sweep_tile(const AstarDev& d, AstarInstDev* Ip, const AstarInstDev& I,
+                                                 AstarTileSmem& sm, const AstarTileGeo& tg, uint32_t n, uint32_t t,
+                                                 uint32_t npar, uint32_t bound, uint32_t* pops) {
+  constexpr uint32_t kStraight = DIAG ? 0x000a000au : 0x00010001u;
+  const uint32_t ts = tg.ts, lts = tg.lts, tid = threadIdx.x, stride = astar_sweep_stride(ts);
+  const uint32_t lsegs = lts - 4u, y = tid >> lsegs, xs = (tid & ((1u << lsegs) - 1u)) << 4;
+  const bool on = y < ts;
+  const uint32_t base = sm.g_min, lim = min(bound, sm.ub);
+  for (uint32_t i = tid; i < n; i += blockDim.x) {
+    const uint2 it = sm.fa[i];
+    const int ix = (int)(it.x & 0xffffu), iy = (int)(it.x >> 16);
+    if (it.y - base < kSweepSpan) sm.vs[((uint32_t)iy - tg.y0 + 1u) * stride + 8u + (uint32_t)ix - tg.x0] = (uint16_t)(it.y - base);
+    else astar_inbox_push(d, Ip, t, npar, it);  // a later visit starts from its g
+  }
+  __syncthreads();
+  uint16_t* row = sm.vs + ((on ? y : 0u) + 1u) * stride + 8u + xs;
+  uint32_t v[8], k1[8];                      // labels; min(old label, window) as astar_pair_below takes it
+  uint32_t cnw[8], cne[8], csw[8], cse[8];   // cost of the diagonal move from each neighbour, 0x8000 = none
+  uint32_t p[8], pa, pb;                     // labels passed on
+  uint32_t items = 0;                        // the thread's cells that are items
+  const int gx = (int)I.gx - (int)(tg.x0 + xs);
+  const uint32_t dyg = (uint32_t)abs((int)(tg.y0 + y) - (int)I.gy);
+  if (on) {
+    astar_load_row(row, p, pa, pb);
+    // blocked bits of columns xs - 1 .. xs + 16 of the rows y - 1, y, y + 1 (outside: blocked)
+    uint32_t bu = ~0u, bc = ~0u, bd = ~0u;
+    auto bits = [&](uint32_t yy) {
+      const uint32_t l = (yy << lts) + xs;
+      uint32_t w = ((sm.blk[l >> 5] >> (l & 31u)) & 0xffffu) << 1;
+      const uint32_t room = tg.tw > xs ? tg.tw - xs : 0u;  // columns inside the grid
+      if (room < 16u) w |= ~0u << (room + 1u);
+      w |= (xs == 0u) ? 1u : ((sm.blk[(l - 1u) >> 5] >> ((l - 1u) & 31u)) & 1u);
+      const bool last = xs + 16u >= tg.tw;
+      w |= (last ? 1u : ((sm.blk[(l + 16u) >> 5] >> ((l + 16u) & 31u)) & 1u)) << 17;
+      return w;
+    };
+    if (y < tg.th) bc = bits(y);
+    if (DIAG) {
+      if (y > 0 && y - 1u < tg.th) bu = bits(y - 1u);
+      if (y + 1u < tg.th) bd = bits(y + 1u);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      uint32_t vv = 0, kk = 0, c0 = 0, c1 = 0, c2 = 0, c3 = 0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int x = 2 * i + h;
+        const uint32_t src = (p[i] >> (16 * h)) & 0xffffu;
+        const bool blocked = (bc >> (x + 1)) & 1u;
+        const uint32_t old = sm.gt[(y << lts) + xs + (uint32_t)x];
+        // the label that stands: below the items' smallest g nothing improves
+        const uint32_t lab = blocked || old < base ? 0u : min(old - base, kSweepInf);
+        const uint32_t hh = DIAG ? 10u * max((uint32_t)abs(x - gx), dyg) + 4u * min((uint32_t)abs(x - gx), dyg)
+                                 : (uint32_t)abs(x - gx) + dyg;
+        const uint32_t win = (lim >= hh && lim - hh >= base) ? min(lim - hh - base + 1u, kSweepSpan) : 0u;
+        const bool item = src != kSweepInf && !blocked;
+        items |= item ? 1u << x : 0u;
+        const uint32_t k = item ? win : min(lab, win);
+        vv |= (item ? src : lab) << (16 * h);
+        kk |= ((k | 0x8000u) - 1u) << (16 * h);
+        if (DIAG) {
+          const bool l = !((bc >> x) & 1u), r = !((bc >> (x + 2)) & 1u);
+          const bool u = !((bu >> (x + 1)) & 1u), w = !((bd >> (x + 1)) & 1u);
+          c0 |= (l && u ? 14u : 0x8000u) << (16 * h);
+          c1 |= (r && u ? 14u : 0x8000u) << (16 * h);
+          c2 |= (l && w ? 14u : 0x8000u) << (16 * h);
+          c3 |= (r && w ? 14u : 0x8000u) << (16 * h);
+        }
+      }
+      v[i] = vv;
+      k1[i] = kk;
+      cnw[i] = c0;
+      cne[i] = c1;
+      csw[i] = c2;
+      cse[i] = c3;
+      // an item whose label no longer lies in the window stays an item: it keeps its label
+      p[i] = astar_pair_below(vv, kk);
+    }
+  }
+  const uint32_t warp = tid >> 5, lane = tid & 31u;
+  const bool warp_on = (warp << 5) < (ts << lsegs);
+  for (uint32_t it = 0;; ++it) {
+    bool any = false;
+    const volatile uint32_t* f = sm.flag[(it + 1u) & 1u] + warp;
+    if (warp_on && (it == 0 || (f[0] | f[1] | f[2]) != 0u)) {
+      for (uint32_t q = 0; q < kSweepsPerBarrier; ++q) {
+        uint32_t up[8], ua, ub2, dn[8], da, db, np[8];
+        bool changed = false;
+        astar_load_row(row - stride, up, ua, ub2);
+        astar_load_row(row + stride, dn, da, db);
+        pa = *reinterpret_cast<const uint32_t*>(row - 2);
+        pb = *reinterpret_cast<const uint32_t*>(row + 16);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          uint32_t a = v[i];
+          a = __viaddmin_u16x2(astar_pair_left(p, i, pa), kStraight, a);
+          a = __viaddmin_u16x2(astar_pair_right(p, i, pb), kStraight, a);
+          a = __viaddmin_u16x2(up[i], kStraight, a);
+          a = __viaddmin_u16x2(dn[i], kStraight, a);
+          if (DIAG) {
+            a = __viaddmin_u16x2(astar_pair_left(up, i, ua), cnw[i], a);
+            a = __viaddmin_u16x2(astar_pair_right(up, i, ub2), cne[i], a);
+            a = __viaddmin_u16x2(astar_pair_left(dn, i, da), csw[i], a);
+            a = __viaddmin_u16x2(astar_pair_right(dn, i, db), cse[i], a);
+          }
+          changed |= a != v[i];
+          v[i] = a;
+          np[i] = astar_pair_below(a, k1[i]);
+        }
+        if (changed) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) p[i] = np[i];
+          *reinterpret_cast<uint4*>(row) = make_uint4(p[0], p[1], p[2], p[3]);
+          *reinterpret_cast<uint4*>(row + 8) = make_uint4(p[4], p[5], p[6], p[7]);
+        }
+        const bool w = __any_sync(GPQ_FULL_MASK, changed);
+        any |= w;
+        if (!w) break;
+      }
+    }
+    if (lane == 0) sm.flag[it & 1u][warp + 1u] = any ? 1u : 0u;
+    if (!__syncthreads_or(any)) break;
+    if (it == kSweepMax) {
+      if (tid == 0) gpq_set_error(&Ip->err, GPQ_ERR_TIMEOUT);
+      break;
+    }
+  }
+  // changed labels: into the global g values; above the window to the open array
+  if (on && y < tg.th) {
+    uint32_t* G = d.gcost + I.cell0 + (uint64_t)(tg.y0 + y) * I.g.width + tg.x0 + xs;
+    const uint32_t ub = sm.ub;
+    uint32_t done = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int x = 2 * i + h;
+        const uint32_t lab = (v[i] >> (16 * h)) & 0xffffu, g = base + lab;
+        const bool passed = ((p[i] >> (16 * h)) & 0xffffu) != kSweepInf;
+        done += passed ? 1u : 0u;
+        if (lab >= kSweepInf || lab == 0u) continue;  // no label, or one that cannot have changed
+        if (g >= sm.gt[(y << lts) + xs + (uint32_t)x]) continue;
+        atomicMin(&G[x], g);
+        if (x == gx && dyg == 0u) {
+          atomicMin(&Ip->ub, g);
+          atomicMin(&sm.ub, g);
+        }
+        if (!passed) {
+          const uint2 itm = make_uint2(astar_pack((int)(tg.x0 + xs) + x, (int)(tg.y0 + y)), g);
+          const uint32_t f = g + astar_hxy(I.g.conn, (int)(tg.x0 + xs) + x, (int)(tg.y0 + y), (int)I.gx, (int)I.gy);
+          if (f <= lim) astar_inbox_push(d, Ip, t, npar, itm);  // beyond the span of this visit's labels
+          else if (f <= ub) astar_open_push(d, Ip, sm, t, itm, f);
+        }
+      }
+    }
+    *pops += done;
+  }
+}
+
+// The moves of this visit's expanded cells into other tiles: cell j of the tile's border.
+__device__ __forceinline__ void astar_send_border(const AstarDev& d, AstarInstDev* Ip, const AstarInstDev& I,
+                                                  const AstarTileSmem& sm, const AstarTileGeo& tg, uint32_t j,
+                                                  uint32_t npar) {
+  uint32_t lx, ly;
+  if (j < 2u * tg.tw) {
+    lx = j >> 1;
+    ly = (j & 1u) ? tg.th - 1u : 0u;
+    if ((j & 1u) && tg.th == 1u) return;
+  } else {
+    j -= 2u * tg.tw;
+    ly = 1u + (j >> 1);
+    lx = (j & 1u) ? tg.tw - 1u : 0u;
+    if (ly + 1u >= tg.th || ((j & 1u) && tg.tw == 1u)) return;
+  }
+  const uint32_t lab = sm.vs[(ly + 1u) * astar_sweep_stride(tg.ts) + 8u + lx];
+  if (lab == kSweepInf) return;
+  const uint32_t g = sm.g_min + lab, conn = I.g.conn;
+  const int x = (int)(tg.x0 + lx), y = (int)(tg.y0 + ly);
+  const uint32_t w = I.g.width, h = I.g.height;
+  for (uint32_t k = 0; k < (conn == 4 ? 4u : 8u); ++k) {
+    const int nx = x + gpq_astar_dx((int)k), ny = y + gpq_astar_dy((int)k);
+    if (nx < 0 || ny < 0 || nx >= (int)w || ny >= (int)h || tg.inside(nx, ny)) continue;
+    if (astar_blocked(d, I, (uint32_t)ny * w + (uint32_t)nx)) continue;
+    if (k >= 4 && (astar_cell_blocked(d, I, sm, tg, nx, y) || astar_cell_blocked(d, I, sm, tg, x, ny))) continue;
+    astar_send(d, Ip, I, make_uint2(astar_pack(nx, ny), g + gpq_astar_cost(conn, (int)k)), npar);
+  }
+}
+
 // Process tile t in round s (one worker).
 template <bool WARP>
 __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, AstarTileSmem& sm,
@@ -404,6 +687,7 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
     sm.pops = 0;
     sm.open_cnt = T->open_cnt;
     sm.open_min = kAstarInf;
+    sm.g_min = kAstarInf;
   }
   wk.sync();
   const uint32_t k_in = min(ldcg_u32(&T->in_cnt[par]), d.in_cap);
@@ -424,12 +708,20 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
     atomicAdd(&d.ctl->visits, 1ull);
   }
   // 0. the tile's g values and blocked bits into shared memory
+  const bool sweeps = astar_sweeps(ts, WARP, blockDim.x);
   for (uint32_t j = wk.tid; j < words; j += wk.n) {
     sm.blk[j] = 0;
-    sm.chg[j] = 0;
+    if (!sweeps) sm.chg[j] = 0;
   }
+  if (sweeps) {
+    uint4* vs4 = reinterpret_cast<uint4*>(sm.vs);
+    const uint4 none = make_uint4(kSweepInf2, kSweepInf2, kSweepInf2, kSweepInf2);
+    for (uint32_t j = wk.tid; j < (ts + 2u) * astar_sweep_stride(ts) / 8u; j += wk.n) vs4[j] = none;
+    if (wk.tid < 20u) (&sm.flag[0][0])[wk.tid] = 0;
+  }
+#pragma unroll 8
   for (uint32_t l = wk.tid; l < ts * ts; l += wk.n) {
-    const uint32_t lx = l % ts, ly = l / ts;
+    const uint32_t lx = l & (ts - 1u), ly = l >> tg.lts;
     sm.gt[l] = (lx < tg.tw && ly < tg.th) ? ldcg_u32(&G[(tg.y0 + ly) * I.g.width + tg.x0 + lx]) : kAstarInf;
   }
   wk.sync();
@@ -500,32 +792,50 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
     T->in_cnt[par] = 0;
     T->queued[par] = 0;
   }
-  // 3. level-by-level expansion of the frontier inside the tile; level i reads buffer
-  //    i % 2 with fill n[i % 3], fills the other buffer and n[(i + 1) % 3], and clears
-  //    n[(i + 2) % 3] (read at level i - 1, filled at level i + 1): one barrier a level
+  // 3. sweeps; the border's moves when all labels stand
   uint32_t pops = 0;
-  for (uint32_t lv = 0;; ++lv) {
-    const uint32_t c3 = lv % 3u;
-    const uint32_t n = min(sm.n[c3], d.frontier_cap);
-    if (n == 0) break;
-    uint2* src = (lv & 1u) ? sm.fb : sm.fa;
-    uint2* dst = (lv & 1u) ? sm.fa : sm.fb;
-    if (wk.tid == 0) sm.n[(c3 + 2u) % 3u] = 0;
-    const uint32_t ipw = I.g.conn == 4 ? 8u : 4u;  // items per warp pass
-    for (uint32_t ib = (wk.tid >> 5) * ipw; ib < n; ib += (wk.n >> 5) * ipw)
-      astar_expand_warp(d, Ip, I, sm, tg, src, ib, n, dst, (c3 + 1u) % 3u, t, npar, bound, &pops);
-    wk.sync();
+  if (sweeps) {
+    const uint32_t n = min(sm.n[0], d.frontier_cap);
+    if (n > 0) {  // the same in every thread
+      uint32_t lo = kAstarInf;
+      for (uint32_t i = wk.tid; i < n; i += wk.n) lo = min(lo, sm.fa[i].y);
+      lo = __reduce_min_sync(GPQ_FULL_MASK, lo);
+      if ((threadIdx.x & 31u) == 0) atomicMin(&sm.g_min, lo);
+      wk.sync();
+      if (I.g.conn == 4) astar_sweep_tile<false>(d, Ip, I, sm, tg, n, t, npar, bound, &pops);
+      else astar_sweep_tile<true>(d, Ip, I, sm, tg, n, t, npar, bound, &pops);
+      const uint32_t border = 2u * (tg.tw + tg.th);
+      for (uint32_t j = wk.tid; j < border; j += wk.n) astar_send_border(d, Ip, I, sm, tg, j, npar);
+    }
+  } else {
+    // list walk: level-by-level expansion of the frontier inside the tile; level i reads
+    // buffer i % 2 with fill n[i % 3], fills the other buffer and n[(i + 1) % 3], and clears
+    // n[(i + 2) % 3] (read at level i - 1, filled at level i + 1): one barrier a level
+    for (uint32_t lv = 0;; ++lv) {
+      const uint32_t c3 = lv % 3u;
+      const uint32_t n = min(sm.n[c3], d.frontier_cap);
+      if (n == 0) break;
+      uint2* src = (lv & 1u) ? sm.fb : sm.fa;
+      uint2* dst = (lv & 1u) ? sm.fa : sm.fb;
+      if (wk.tid == 0) sm.n[(c3 + 2u) % 3u] = 0;
+      const uint32_t ipw = I.g.conn == 4 ? 8u : 4u;  // items per warp pass
+      for (uint32_t ib = (wk.tid >> 5) * ipw; ib < n; ib += (wk.n >> 5) * ipw)
+        astar_expand_warp(d, Ip, I, sm, tg, src, ib, n, dst, (c3 + 1u) % 3u, t, npar, bound, &pops);
+      wk.sync();
+    }
+    // 4. send the moves into other tiles
+    {
+      const uint32_t nob = min(sm.ob_n, astar_outbox_cap(ts));
+      for (uint32_t i = wk.tid; i < nob; i += wk.n) astar_send(d, Ip, I, sm.ob[i], npar);
+    }
   }
-  // 4. send the moves into other tiles
-  {
-    const uint32_t nob = min(sm.ob_n, astar_outbox_cap(ts));
-    for (uint32_t i = wk.tid; i < nob; i += wk.n) astar_send(d, Ip, I, sm.ob[i], npar);
-  }
-  // 5. merge the tile's g values back
-  for (uint32_t l = wk.tid; l < ts * ts; l += wk.n) {
-    if ((sm.chg[l >> 5] >> (l & 31u)) & 1u) {
-      const uint32_t lx = l % ts, ly = l / ts;
-      atomicMin(&G[(tg.y0 + ly) * I.g.width + tg.x0 + lx], sm.gt[l]);
+  // 5. list walk: merge the tile's g values back
+  if (!sweeps) {
+    for (uint32_t l = wk.tid; l < ts * ts; l += wk.n) {
+      if ((sm.chg[l >> 5] >> (l & 31u)) & 1u) {
+        const uint32_t lx = l & (ts - 1u), ly = l >> tg.lts;
+        atomicMin(&G[(tg.y0 + ly) * I.g.width + tg.x0 + lx], sm.gt[l]);
+      }
     }
   }
   pops = warp_sum_u32(pops);
@@ -577,27 +887,22 @@ static __device__ void astar_window_step(const AstarDev& d, uint32_t i, uint32_t
 // astar_worker_smem_bytes(ts, frontier_cap) per worker (per warp when WARP).
 static constexpr uint32_t kAstarMaxWorkers = 8;  // 256 threads / 32
 
-__host__ __device__ inline size_t astar_worker_smem_bytes(uint32_t ts, uint32_t frontier_cap) {
-  return (astar_smem_bytes(ts, frontier_cap) + 15u) & ~(size_t)15u;
+__host__ __device__ inline size_t astar_worker_smem_bytes(uint32_t ts, uint32_t frontier_cap, bool warp, uint32_t block) {
+  return (astar_smem_bytes(ts, frontier_cap, warp, block) + 15u) & ~(size_t)15u;
 }
 
 // Rounds s0, s0 + 1, ... until every instance is done, or until `step_rounds` rounds ran
 // (0 = no limit): a resident session resumes at the next round in its next launch.
 template <bool WARP>
-static __global__ void __launch_bounds__(256) astar_persistent_kernel(AstarDev d, uint32_t s0, uint32_t step_rounds) {
+static __global__ void __launch_bounds__(256, 2) astar_persistent_kernel(AstarDev d, uint32_t s0, uint32_t step_rounds) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ AstarTileSmem sms[kAstarMaxWorkers];
   __shared__ uint32_t s_t;
   const AstarWorker<WARP> wk;
   AstarTileSmem& sm = sms[wk.id];
   if (wk.tid == 0) {
-    unsigned char* base = smem_raw + (size_t)wk.id * astar_worker_smem_bytes(d.ts, d.frontier_cap);
-    sm.fa = reinterpret_cast<uint2*>(base);
-    sm.fb = sm.fa + d.frontier_cap;
-    sm.ob = sm.fb + d.frontier_cap;
-    sm.gt = reinterpret_cast<uint32_t*>(sm.ob + astar_outbox_cap(d.ts));
-    sm.blk = sm.gt + d.ts * d.ts;
-    sm.chg = sm.blk + d.ts * d.ts / 32;
+    astar_smem_carve(sm, smem_raw + (size_t)wk.id * astar_worker_smem_bytes(d.ts, d.frontier_cap, WARP, blockDim.x),
+                     d.ts, d.frontier_cap, WARP);
   }
   __syncthreads();
   const unsigned long long nb = gridDim.x;
