@@ -18,7 +18,8 @@
 //     the next round.
 //   * phase W: an instance whose tiles sent nothing for the next round has drained its
 //     window; the window moves to [min f of its open arrays, + delta], or the instance
-//     is done when that minimum exceeds UB.
+//     is done when that minimum exceeds UB.  The CTA that makes the instance's last visit
+//     of a round decides this, so a round has one grid barrier.
 //
 // Work items are 8 bytes (y << 16 | x, g); f = g + h(x, y) is recomputed, so the hot loop
 // needs no division.  With a consistent
@@ -44,7 +45,8 @@ struct AstarInstDev {
   uint32_t tiles_x, tiles_y;
   uint32_t ub;         // best goal cost found so far
   uint32_t bound;      // window: items with f <= bound are expanded
-  uint32_t active_next;
+  uint32_t active[2];  // active tiles of the round with this parity
+  uint32_t visited;    // of the current round's active tiles
   uint32_t done;
   uint32_t err;
   uint32_t windows;
@@ -65,8 +67,8 @@ struct AstarTileDev {
 
 // Control words of one launch.
 struct AstarCtl {
-  uint32_t al_cnt[2];
-  uint32_t work[2];
+  uint32_t al_cnt[3];  // active tiles by round mod 3: read in this round, filled for the next, cleared
+  uint32_t work[3];    // tiles handed out beyond each worker's first
   uint32_t err;
   uint32_t rounds;
   unsigned long long bar;
@@ -114,24 +116,27 @@ __device__ __forceinline__ uint32_t astar_hxy(uint32_t conn, int x, int y, int g
 
 __device__ __forceinline__ uint32_t astar_pack(int x, int y) { return ((uint32_t)y << 16) | (uint32_t)x; }
 
-// Put tile t on the active list of round parity `par` (once per round).
-__device__ __forceinline__ void astar_activate(const AstarDev& d, uint32_t t, uint32_t par, bool count) {
+// Put tile t on the active list of a round (once per round).
+__device__ __forceinline__ void astar_activate(const AstarDev& d, AstarInstDev* Ip, uint32_t t, uint32_t round) {
+  const uint32_t par = round & 1u;
   if (atomicExch(&d.tiles[t].queued[par], 1u) == 0u) {
-    const uint32_t pos = atomicAdd(&d.ctl->al_cnt[par], 1u);
+    const uint32_t pos = atomicAdd(&d.ctl->al_cnt[round % 3u], 1u);
     d.al[(size_t)par * d.n_tiles + pos] = t;
-    if (count) atomicAdd(&d.inst[d.tiles[t].inst].active_next, 1u);
+    atomicAdd(&Ip->active[par], 1u);
   }
 }
 
-__device__ __forceinline__ void astar_inbox_push(const AstarDev& d, AstarInstDev* Ip, uint32_t t, uint32_t par,
+// An item into a tile's inbox of a round.
+__device__ __forceinline__ void astar_inbox_push(const AstarDev& d, AstarInstDev* Ip, uint32_t t, uint32_t round,
                                                  uint2 it) {
+  const uint32_t par = round & 1u;
   const uint32_t pos = atomicAdd(&d.tiles[t].in_cnt[par], 1u);
   if (pos < d.in_cap) {
     d.inbox[((size_t)par * d.n_tiles + t) * d.in_cap + pos] = it;
   } else {
     gpq_set_error(&Ip->err, GPQ_ERR_INSERT_FULL);
   }
-  astar_activate(d, t, par, true);
+  astar_activate(d, Ip, t, round);
 }
 
 // Shared state of the CTA working on one tile.  While a CTA holds a tile, the tile's g
@@ -153,6 +158,8 @@ struct AstarTileSmem {
   uint32_t open_min;
   uint32_t open_cnt;
   uint32_t g_min;  // of the items to expand
+  uint32_t last;   // this visit was its instance's last of the round
+  uint32_t out_n[9], out_base[9];  // sweeps: moves into each neighbour tile, their place in its inbox
   unsigned long long pops;
   uint32_t scan[33];
 };
@@ -237,12 +244,12 @@ struct AstarWorker {
 // Frontier push: into the shared buffer, or (when it is full) into the tile's own inbox
 // for the next round.
 __device__ __forceinline__ void astar_frontier_push(const AstarDev& d, AstarInstDev* Ip, AstarTileSmem& sm,
-                                                    uint2* buf, uint32_t which, uint32_t t, uint32_t npar, uint2 it) {
+                                                    uint2* buf, uint32_t which, uint32_t t, uint32_t next_round, uint2 it) {
   const uint32_t pos = atomicAdd(&sm.n[which], 1u);
   if (pos < d.frontier_cap) {
     buf[pos] = it;
   } else {
-    astar_inbox_push(d, Ip, t, npar, it);
+    astar_inbox_push(d, Ip, t, next_round, it);
   }
 }
 
@@ -269,7 +276,7 @@ __device__ __forceinline__ bool astar_cell_blocked(const AstarDev& d, const Asta
 // A move into another tile: lower the cell's global g (the filter), and when that
 // improves it, send the item to the owning tile's inbox for the next round.
 __device__ __forceinline__ void astar_send(const AstarDev& d, AstarInstDev* Ip, const AstarInstDev& I, uint2 it,
-                                           uint32_t npar) {
+                                           uint32_t next_round) {
   const int x = (int)(it.x & 0xffffu), y = (int)(it.x >> 16);
   const uint32_t ng = it.y;
   if (ng >= atomicMin(&d.gcost[I.cell0 + (uint32_t)y * I.g.width + (uint32_t)x], ng)) return;
@@ -277,7 +284,7 @@ __device__ __forceinline__ void astar_send(const AstarDev& d, AstarInstDev* Ip, 
   if (x == (int)I.gx && y == (int)I.gy) atomicMin(&Ip->ub, ng);
   if (nf > ldcg_u32(&Ip->ub)) return;
   const uint32_t nt = I.tile0 + ((uint32_t)y >> d.lts) * I.tiles_x + ((uint32_t)x >> d.lts);
-  astar_inbox_push(d, Ip, nt, npar, it);
+  astar_inbox_push(d, Ip, nt, next_round, it);
 }
 
 // Expand frontier items src[ib .. ib + 32 / M) with one warp, one lane per (item, move):
@@ -288,7 +295,7 @@ __device__ __forceinline__ void astar_send(const AstarDev& d, AstarInstDev* Ip, 
 __device__ __forceinline__ void astar_expand_warp(const AstarDev& d, AstarInstDev* Ip, const AstarInstDev& I,
                                                   AstarTileSmem& sm, const AstarTileGeo& tg, const uint2* src,
                                                   uint32_t ib, uint32_t n, uint2* next, uint32_t which, uint32_t t,
-                                                  uint32_t npar, uint32_t bound, uint32_t* pops) {
+                                                  uint32_t next_round, uint32_t bound, uint32_t* pops) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t lt = (1u << lane) - 1u;
   const uint32_t conn = I.g.conn;
@@ -346,7 +353,7 @@ __device__ __forceinline__ void astar_expand_warp(const AstarDev& d, AstarInstDe
     if (kind == 1u) {
       const uint32_t pos = base + __popc(mf & lt);
       if (pos < d.frontier_cap) next[pos] = child;
-      else astar_inbox_push(d, Ip, t, npar, child);  // full: the tile's own next round
+      else astar_inbox_push(d, Ip, t, next_round, child);  // full: the tile's own next round
     }
   }
   const uint32_t mx = __ballot_sync(GPQ_FULL_MASK, kind == 4u);
@@ -358,7 +365,7 @@ __device__ __forceinline__ void astar_expand_warp(const AstarDev& d, AstarInstDe
     if (kind == 4u) {
       const uint32_t pos = base + __popc(mx & lt);
       if (pos < astar_outbox_cap(tg.ts)) sm.ob[pos] = child;
-      else astar_send(d, Ip, I, child, npar);  // full: send now
+      else astar_send(d, Ip, I, child, next_round);  // full: send now
     }
   }
   const uint32_t mo = __ballot_sync(GPQ_FULL_MASK, kind == 2u);
@@ -476,7 +483,7 @@ __device__ __forceinline__ void astar_load_row(const uint16_t* row, uint32_t* p,
 template <bool DIAG>
 __device__ __forceinline__ void astar_sweep_tile(const AstarDev& d, AstarInstDev* Ip, const AstarInstDev& I,
                                                  AstarTileSmem& sm, const AstarTileGeo& tg, uint32_t n, uint32_t t,
-                                                 uint32_t npar, uint32_t bound, uint32_t* pops) {
+                                                 uint32_t next_round, uint32_t bound, uint32_t* pops) {
   constexpr uint32_t kStraight = DIAG ? 0x000a000au : 0x00010001u;
   const uint32_t ts = tg.ts, lts = tg.lts, tid = threadIdx.x, stride = astar_sweep_stride(ts);
   const uint32_t lsegs = lts - 4u, y = tid >> lsegs, xs = (tid & ((1u << lsegs) - 1u)) << 4;
@@ -486,7 +493,7 @@ __device__ __forceinline__ void astar_sweep_tile(const AstarDev& d, AstarInstDev
     const uint2 it = sm.fa[i];
     const int ix = (int)(it.x & 0xffffu), iy = (int)(it.x >> 16);
     if (it.y - base < kSweepSpan) sm.vs[((uint32_t)iy - tg.y0 + 1u) * stride + 8u + (uint32_t)ix - tg.x0] = (uint16_t)(it.y - base);
-    else astar_inbox_push(d, Ip, t, npar, it);  // a later visit starts from its g
+    else astar_inbox_push(d, Ip, t, next_round, it);  // a later visit starts from its g
   }
   __syncthreads();
   uint16_t* row = sm.vs + ((on ? y : 0u) + 1u) * stride + 8u + xs;
@@ -624,7 +631,7 @@ __device__ __forceinline__ void astar_sweep_tile(const AstarDev& d, AstarInstDev
         if (!passed) {
           const uint2 itm = make_uint2(astar_pack((int)(tg.x0 + xs) + x, (int)(tg.y0 + y)), g);
           const uint32_t f = g + astar_hxy(I.g.conn, (int)(tg.x0 + xs) + x, (int)(tg.y0 + y), (int)I.gx, (int)I.gy);
-          if (f <= lim) astar_inbox_push(d, Ip, t, npar, itm);  // beyond the span of this visit's labels
+          if (f <= lim) astar_inbox_push(d, Ip, t, next_round, itm);  // beyond the span of this visit's labels
           else if (f <= ub) astar_open_push(d, Ip, sm, t, itm, f);
         }
       }
@@ -633,32 +640,122 @@ __device__ __forceinline__ void astar_sweep_tile(const AstarDev& d, AstarInstDev
   }
 }
 
-// The moves of this visit's expanded cells into other tiles: cell j of the tile's border.
+// The moves of this visit's expanded cells into other tiles (all threads; a tile's border
+// has at most 4 * 64 - 4 cells).  A cell's moves lower the global g values together, then
+// the improving ones are counted by neighbour tile, one thread per neighbour reserves their
+// place in its inbox, and all are stored: three round trips whatever the number of moves,
+// where each move by itself took five one after another.
+template <bool DIAG>
 __device__ __forceinline__ void astar_send_border(const AstarDev& d, AstarInstDev* Ip, const AstarInstDev& I,
-                                                  const AstarTileSmem& sm, const AstarTileGeo& tg, uint32_t j,
-                                                  uint32_t npar) {
-  uint32_t lx, ly;
-  if (j < 2u * tg.tw) {
-    lx = j >> 1;
-    ly = (j & 1u) ? tg.th - 1u : 0u;
-    if ((j & 1u) && tg.th == 1u) return;
-  } else {
-    j -= 2u * tg.tw;
-    ly = 1u + (j >> 1);
-    lx = (j & 1u) ? tg.tw - 1u : 0u;
-    if (ly + 1u >= tg.th || ((j & 1u) && tg.tw == 1u)) return;
+                                                  AstarTileSmem& sm, const AstarTileGeo& tg, uint32_t next_round) {
+  constexpr uint32_t M = DIAG ? 8u : 4u;
+  const uint32_t w = I.g.width, h = I.g.height, border = 2u * (tg.tw + tg.th);
+  const uint32_t npar = next_round & 1u;
+  for (uint32_t j0 = 0; j0 < border; j0 += blockDim.x) {
+    if (threadIdx.x < 9u) sm.out_n[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t j = j0 + threadIdx.x;
+    uint32_t lx, ly;
+    bool ok = j < border;
+    if (j < 2u * tg.tw) {  // the top and the bottom row, then the sides without their corners
+      lx = j >> 1;
+      ly = (j & 1u) ? tg.th - 1u : 0u;
+      if ((j & 1u) && tg.th == 1u) ok = false;
+    } else {
+      const uint32_t jj = j - 2u * tg.tw;
+      ly = 1u + (jj >> 1);
+      lx = (jj & 1u) ? tg.tw - 1u : 0u;
+      if (ly + 1u >= tg.th || ((jj & 1u) && tg.tw == 1u)) ok = false;
+    }
+    const uint32_t lab = ok ? sm.vs[(ly + 1u) * astar_sweep_stride(tg.ts) + 8u + lx] : kSweepInf;
+    ok = ok && lab != kSweepInf;
+    const int x = (int)(tg.x0 + lx), y = (int)(tg.y0 + ly);
+    const uint32_t g = sm.g_min + lab;
+    const uint32_t ub = ok ? min(sm.ub, ldcg_u32(&Ip->ub)) : 0u;
+    uint32_t old[M];
+    bool go[M];
+#pragma unroll
+    for (uint32_t k = 0; k < M; ++k) {
+      const int nx = x + gpq_astar_dx((int)k), ny = y + gpq_astar_dy((int)k);
+      go[k] = ok && nx >= 0 && ny >= 0 && nx < (int)w && ny < (int)h && !tg.inside(nx, ny) &&
+              !astar_blocked(d, I, (uint32_t)ny * w + (uint32_t)nx) &&
+              (k < 4 || (!astar_cell_blocked(d, I, sm, tg, nx, y) && !astar_cell_blocked(d, I, sm, tg, x, ny)));
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < M; ++k) {
+      const uint32_t c = (uint32_t)(y + gpq_astar_dy((int)k)) * w + (uint32_t)(x + gpq_astar_dx((int)k));
+      old[k] = 0;
+      if (go[k]) old[k] = atomicMin(&d.gcost[I.cell0 + c], g + gpq_astar_cost(DIAG ? 8 : 4, (int)k));
+    }
+    uint32_t place[M];  // neighbour tile << 16 | position among the moves into it
+#pragma unroll
+    for (uint32_t k = 0; k < M; ++k) {
+      const int nx = x + gpq_astar_dx((int)k), ny = y + gpq_astar_dy((int)k);
+      const uint32_t ng = g + gpq_astar_cost(DIAG ? 8 : 4, (int)k);
+      place[k] = ~0u;
+      if (!go[k] || ng >= old[k]) continue;
+      if (nx == (int)I.gx && ny == (int)I.gy) atomicMin(&Ip->ub, ng);
+      if (ng + astar_hxy(I.g.conn, nx, ny, (int)I.gx, (int)I.gy) > ub) continue;
+      const uint32_t dir = (nx < (int)tg.x0 ? 0u : nx >= (int)(tg.x0 + tg.ts) ? 2u : 1u) +
+                           (ny < (int)tg.y0 ? 0u : ny >= (int)(tg.y0 + tg.ts) ? 6u : 3u);
+      place[k] = (dir << 16) | atomicAdd(&sm.out_n[dir], 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x < 9u && sm.out_n[threadIdx.x]) {
+      const uint32_t nt = I.tile0 + ((tg.y0 >> tg.lts) + threadIdx.x / 3u - 1u) * I.tiles_x + (tg.x0 >> tg.lts) +
+                          threadIdx.x % 3u - 1u;
+      sm.out_base[threadIdx.x] = atomicAdd(&d.tiles[nt].in_cnt[npar], sm.out_n[threadIdx.x]);
+      astar_activate(d, Ip, nt, next_round);
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t k = 0; k < M; ++k) {
+      if (place[k] == ~0u) continue;
+      const int nx = x + gpq_astar_dx((int)k), ny = y + gpq_astar_dy((int)k);
+      const uint32_t nt = I.tile0 + ((uint32_t)ny >> tg.lts) * I.tiles_x + ((uint32_t)nx >> tg.lts);
+      const uint32_t pos = sm.out_base[place[k] >> 16] + (place[k] & 0xffffu);
+      if (pos < d.in_cap)
+        d.inbox[((size_t)npar * d.n_tiles + nt) * d.in_cap + pos] =
+            make_uint2(astar_pack(nx, ny), g + gpq_astar_cost(DIAG ? 8 : 4, (int)k));
+      else
+        gpq_set_error(&Ip->err, GPQ_ERR_INSERT_FULL);
+    }
+    __syncthreads();
   }
-  const uint32_t lab = sm.vs[(ly + 1u) * astar_sweep_stride(tg.ts) + 8u + lx];
-  if (lab == kSweepInf) return;
-  const uint32_t g = sm.g_min + lab, conn = I.g.conn;
-  const int x = (int)(tg.x0 + lx), y = (int)(tg.y0 + ly);
-  const uint32_t w = I.g.width, h = I.g.height;
-  for (uint32_t k = 0; k < (conn == 4 ? 4u : 8u); ++k) {
-    const int nx = x + gpq_astar_dx((int)k), ny = y + gpq_astar_dy((int)k);
-    if (nx < 0 || ny < 0 || nx >= (int)w || ny >= (int)h || tg.inside(nx, ny)) continue;
-    if (astar_blocked(d, I, (uint32_t)ny * w + (uint32_t)nx)) continue;
-    if (k >= 4 && (astar_cell_blocked(d, I, sm, tg, nx, y) || astar_cell_blocked(d, I, sm, tg, x, ny))) continue;
-    astar_send(d, Ip, I, make_uint2(astar_pack(nx, ny), g + gpq_astar_cost(conn, (int)k)), npar);
+}
+
+// Phase W for one instance, by the worker that made the instance's last visit of the round,
+// when its tiles sent nothing for the next one: the drained window moves on, or the
+// instance ends.  sm.open_min is all ones on entry.
+template <bool WARP>
+__device__ __forceinline__ void astar_window_step(const AstarDev& d, AstarInstDev* Ip, uint32_t next_round,
+                                                  AstarTileSmem& sm, const AstarWorker<WARP>& wk) {
+  const uint32_t nt = Ip->tiles_x * Ip->tiles_y, t0 = Ip->tile0;
+  uint32_t m = kAstarInf;
+  for (uint32_t j = wk.tid; j < nt; j += wk.n) {
+    const AstarTileDev* T = d.tiles + t0 + j;
+    const uint32_t oc = ldcg_u32(&T->open_cnt), om = ldcg_u32(&T->open_min);
+    if (oc) m = min(m, om);
+  }
+  m = warp_min_u32(m);
+  if ((threadIdx.x & 31u) == 0) atomicMin(&sm.open_min, m);
+  wk.sync();
+  m = sm.open_min;
+  const uint32_t ub = ldcg_u32(&Ip->ub);
+  if (m == kAstarInf || m > ub) {
+    if (wk.tid == 0) Ip->done = 1;
+    return;
+  }
+  uint32_t bound = m + Ip->delta;
+  if (bound < m || bound > ub) bound = ub;
+  if (wk.tid == 0) {
+    Ip->bound = bound;
+    Ip->windows += 1;
+  }
+  for (uint32_t j = wk.tid; j < nt; j += wk.n) {
+    const AstarTileDev* T = d.tiles + t0 + j;
+    const uint32_t oc = ldcg_u32(&T->open_cnt), om = ldcg_u32(&T->open_min);
+    if (oc && om <= bound) astar_activate(d, Ip, t0 + j, next_round);
   }
 }
 
@@ -666,7 +763,7 @@ __device__ __forceinline__ void astar_send_border(const AstarDev& d, AstarInstDe
 template <bool WARP>
 __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, AstarTileSmem& sm,
                                    const AstarWorker<WARP>& wk) {
-  const uint32_t par = s & 1u, npar = par ^ 1u;
+  const uint32_t par = s & 1u, next_round = s + 1u;
   AstarTileDev* T = d.tiles + t;
   AstarInstDev* Ip = d.inst + T->inst;
   const AstarInstDev I = *Ip;  // static fields; ub/bound are read through Ip
@@ -719,10 +816,17 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
     for (uint32_t j = wk.tid; j < (ts + 2u) * astar_sweep_stride(ts) / 8u; j += wk.n) vs4[j] = none;
     if (wk.tid < 20u) (&sm.flag[0][0])[wk.tid] = 0;
   }
-#pragma unroll 8
-  for (uint32_t l = wk.tid; l < ts * ts; l += wk.n) {
-    const uint32_t lx = l & (ts - 1u), ly = l >> tg.lts;
-    sm.gt[l] = (lx < tg.tw && ly < tg.th) ? ldcg_u32(&G[(tg.y0 + ly) * I.g.width + tg.x0 + lx]) : kAstarInf;
+  // (sixteen loads of a thread in flight at a time: the copy is a round trip to L2 otherwise repeated)
+  for (uint32_t l0 = wk.tid; l0 < ts * ts; l0 += 16u * wk.n) {
+    uint32_t g[16];
+#pragma unroll
+    for (uint32_t q = 0; q < 16; ++q) {
+      const uint32_t l = l0 + q * wk.n, lx = l & (ts - 1u), ly = l >> tg.lts;
+      g[q] = (l < ts * ts && lx < tg.tw && ly < tg.th) ? ldcg_u32(&G[(tg.y0 + ly) * I.g.width + tg.x0 + lx]) : kAstarInf;
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < 16; ++q)
+      if (l0 + q * wk.n < ts * ts) sm.gt[l0 + q * wk.n] = g[q];
   }
   wk.sync();
   {
@@ -755,7 +859,7 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
         if (sm.gt[tg.local(x, y)] == it.y) {
           f = it.y + astar_hxy(I.g.conn, x, y, (int)I.gx, (int)I.gy);
           if (f <= ub) {
-            if (f <= bound) astar_frontier_push(d, Ip, sm, sm.fa, 0, t, npar, it);
+            if (f <= bound) astar_frontier_push(d, Ip, sm, sm.fa, 0, t, next_round, it);
             else keep = 1;
           }
         }
@@ -783,7 +887,7 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
       if (sm.gt[tg.local(x, y)] != it.y) continue;
       const uint32_t f = it.y + astar_hxy(I.g.conn, x, y, (int)I.gx, (int)I.gy);
       if (f > ub) continue;
-      if (f <= bound) astar_frontier_push(d, Ip, sm, sm.fa, 0, t, npar, it);
+      if (f <= bound) astar_frontier_push(d, Ip, sm, sm.fa, 0, t, next_round, it);
       else astar_open_push(d, Ip, sm, t, it, f);
     }
   }
@@ -802,10 +906,13 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
       lo = __reduce_min_sync(GPQ_FULL_MASK, lo);
       if ((threadIdx.x & 31u) == 0) atomicMin(&sm.g_min, lo);
       wk.sync();
-      if (I.g.conn == 4) astar_sweep_tile<false>(d, Ip, I, sm, tg, n, t, npar, bound, &pops);
-      else astar_sweep_tile<true>(d, Ip, I, sm, tg, n, t, npar, bound, &pops);
-      const uint32_t border = 2u * (tg.tw + tg.th);
-      for (uint32_t j = wk.tid; j < border; j += wk.n) astar_send_border(d, Ip, I, sm, tg, j, npar);
+      if (I.g.conn == 4) {
+        astar_sweep_tile<false>(d, Ip, I, sm, tg, n, t, next_round, bound, &pops);
+        astar_send_border<false>(d, Ip, I, sm, tg, next_round);
+      } else {
+        astar_sweep_tile<true>(d, Ip, I, sm, tg, n, t, next_round, bound, &pops);
+        astar_send_border<true>(d, Ip, I, sm, tg, next_round);
+      }
     }
   } else {
     // list walk: level-by-level expansion of the frontier inside the tile; level i reads
@@ -820,13 +927,13 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
       if (wk.tid == 0) sm.n[(c3 + 2u) % 3u] = 0;
       const uint32_t ipw = I.g.conn == 4 ? 8u : 4u;  // items per warp pass
       for (uint32_t ib = (wk.tid >> 5) * ipw; ib < n; ib += (wk.n >> 5) * ipw)
-        astar_expand_warp(d, Ip, I, sm, tg, src, ib, n, dst, (c3 + 1u) % 3u, t, npar, bound, &pops);
+        astar_expand_warp(d, Ip, I, sm, tg, src, ib, n, dst, (c3 + 1u) % 3u, t, next_round, bound, &pops);
       wk.sync();
     }
     // 4. send the moves into other tiles
     {
       const uint32_t nob = min(sm.ob_n, astar_outbox_cap(ts));
-      for (uint32_t i = wk.tid; i < nob; i += wk.n) astar_send(d, Ip, I, sm.ob[i], npar);
+      for (uint32_t i = wk.tid; i < nob; i += wk.n) astar_send(d, Ip, I, sm.ob[i], next_round);
     }
   }
   // 5. list walk: merge the tile's g values back
@@ -846,41 +953,20 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
     T->open_cnt = oc;
     T->open_min = oc ? sm.open_min : kAstarInf;
     if (sm.pops) atomicAdd(&Ip->pops, sm.pops);
+    // the instance's last visit of the round: every send and open array of the round stands
+    __threadfence();
+    const uint32_t last = atomicAdd(&Ip->visited, 1u) + 1u == ldcg_u32(&Ip->active[par]) ? 1u : 0u;
+    __threadfence();
+    sm.last = last;
+    sm.open_min = kAstarInf;
+    if (last) {
+      Ip->visited = 0;
+      Ip->active[par] = 0;
+    }
   }
   wk.sync();
-}
-
-// Phase W for one instance (one warp): a drained window moves on, or the instance ends.
-static __device__ void astar_window_step(const AstarDev& d, uint32_t i, uint32_t npar) {
-  AstarInstDev* Ip = d.inst + i;
-  const uint32_t lane = threadIdx.x & 31u;
-  if (ldcg_u32(&Ip->done)) return;
-  const uint32_t a = ldcg_u32(&Ip->active_next);
-  __syncwarp();
-  if (lane == 0) Ip->active_next = 0;
-  if (a > 0) return;
-  const uint32_t nt = Ip->tiles_x * Ip->tiles_y, t0 = Ip->tile0;
-  uint32_t m = kAstarInf;
-  for (uint32_t j = lane; j < nt; j += 32) {
-    const AstarTileDev* T = d.tiles + t0 + j;
-    if (ldcg_u32(&T->open_cnt)) m = min(m, ldcg_u32(&T->open_min));
-  }
-  m = warp_min_u32(m);
-  const uint32_t ub = ldcg_u32(&Ip->ub);
-  if (m == kAstarInf || m > ub) {
-    if (lane == 0) Ip->done = 1;
-    return;
-  }
-  uint32_t bound = m + Ip->delta;
-  if (bound < m || bound > ub) bound = ub;
-  if (lane == 0) {
-    Ip->bound = bound;
-    Ip->windows += 1;
-  }
-  for (uint32_t j = lane; j < nt; j += 32) {
-    AstarTileDev* T = d.tiles + t0 + j;
-    if (ldcg_u32(&T->open_cnt) && ldcg_u32(&T->open_min) <= bound) astar_activate(d, t0 + j, npar, false);
-  }
+  if (sm.last && ldcg_u32(&Ip->active[next_round & 1u]) == 0u) astar_window_step<WARP>(d, Ip, next_round, sm, wk);
+  wk.sync();
 }
 
 // The persistent search loop over all instances.  Dynamic shared memory: one slice of
@@ -907,37 +993,33 @@ static __global__ void __launch_bounds__(256, 2) astar_persistent_kernel(AstarDe
   __syncthreads();
   const unsigned long long nb = gridDim.x;
   unsigned long long bar_target = 0;
-  const uint32_t warps_total = gridDim.x * (blockDim.x >> 5);
-  const uint32_t gwarp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const uint32_t per_cta = WARP ? blockDim.x >> 5 : 1u;
+  const uint32_t workers = gridDim.x * per_cta, me = blockIdx.x * per_cta + wk.id;
   for (uint32_t s = s0;; ++s) {
-    const uint32_t par = s & 1u, npar = par ^ 1u;
-    const uint32_t n = ldcg_u32(&d.ctl->al_cnt[par]);
-    for (;;) {
-      uint32_t j;
+    const uint32_t par = s & 1u, cur = s % 3u, nxt = (s + 1u) % 3u, old = (s + 2u) % 3u;
+    const uint32_t n = ldcg_u32(&d.ctl->al_cnt[cur]);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // last read in round s - 1, filled again in round s + 1
+      d.ctl->al_cnt[old] = 0;
+      d.ctl->work[old] = 0;
+      d.ctl->rounds = s + 1;
+    }
+    // each worker's first tile goes by its number, later ones from a counter
+    for (uint32_t j = me; j < n;) {
+      astar_process_tile<WARP>(d, d.al[(size_t)par * d.n_tiles + j], s, sm, wk);
+      if (n <= workers) break;
       if (WARP) {
-        j = 0;
-        if (wk.tid == 0) j = atomicAdd(&d.ctl->work[par], 1u);
+        if (wk.tid == 0) j = workers + atomicAdd(&d.ctl->work[cur], 1u);
         j = __shfl_sync(GPQ_FULL_MASK, j, 0);
       } else {
-        if (threadIdx.x == 0) s_t = atomicAdd(&d.ctl->work[par], 1u);
+        if (threadIdx.x == 0) s_t = workers + atomicAdd(&d.ctl->work[cur], 1u);
         __syncthreads();
         j = s_t;
         __syncthreads();
       }
-      if (j >= n) break;
-      astar_process_tile<WARP>(d, d.al[(size_t)par * d.n_tiles + j], s, sm, wk);
     }
     bar_target += nb;
     if (!grid_barrier(&d.ctl->bar, bar_target, d.spin_limit, &d.ctl->err)) return;
-    for (uint32_t i = gwarp; i < d.n_inst; i += warps_total) astar_window_step(d, i, npar);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      d.ctl->al_cnt[par] = 0;
-      d.ctl->work[par] = 0;
-      d.ctl->rounds = s + 1;
-    }
-    bar_target += nb;
-    if (!grid_barrier(&d.ctl->bar, bar_target, d.spin_limit, &d.ctl->err)) return;
-    if (ldcg_u32(&d.ctl->al_cnt[npar]) == 0 || ldcg_u32(&d.ctl->err) != 0) break;
+    if (ldcg_u32(&d.ctl->al_cnt[nxt]) == 0 || ldcg_u32(&d.ctl->err) != 0) break;
     if (d.max_rounds && s + 1 >= d.max_rounds) {
       if (blockIdx.x == 0 && threadIdx.x == 0) gpq_set_error(&d.ctl->err, GPQ_ERR_TIMEOUT);
       break;
@@ -971,19 +1053,20 @@ static __global__ void astar_bitmap_kernel(const AstarInstDev* inst, uint32_t n_
 }
 
 // Initial state of instances list[0, n) (all instances when list == nullptr): g = inf
-// (done by a memset), g[start] = 0, the start item in the start tile's inbox of round
-// parity par, the start tile on that round's active list.
-static __global__ void astar_init_kernel(AstarDev d, const uint32_t* list, uint32_t n, uint32_t par) {
+// (done by a memset), g[start] = 0, the start item in the start tile's inbox of `round`,
+// the start tile on that round's active list.
+static __global__ void astar_init_kernel(AstarDev d, const uint32_t* list, uint32_t n, uint32_t round) {
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const uint32_t i = list ? list[j] : j;
   AstarInstDev& I = d.inst[i];
   d.gcost[I.cell0 + I.g.start] = 0;
   const uint32_t t = astar_tile_of(d, I, I.g.start);
+  const uint32_t par = round & 1u;
   d.tiles[t].in_cnt[par] = 1;
   d.inbox[((size_t)par * d.n_tiles + t) * d.in_cap] =
       make_uint2(astar_pack((int)(I.g.start % I.g.width), (int)(I.g.start / I.g.width)), 0);
-  astar_activate(d, t, par, false);
+  astar_activate(d, &I, t, round);
 }
 
 // Tile records of instances list[0, n) (all when list == nullptr): one block per instance.

@@ -127,7 +127,7 @@ gpq_status flush_pending(gpq_astar_session* s, cudaStream_t st) {
     astar_bitmap_list_kernel<<<dim3(bx, nj), 256, 0, st>>>(s->inst, s->list + j0, s->blk);
   }
   astar_tiles_init_kernel<<<std::min<uint32_t>(n, 4096), 128, 0, st>>>(d, s->list, n);
-  astar_init_kernel<<<(n + 127) / 128, 128, 0, st>>>(d, s->list, n, s->next_round & 1u);
+  astar_init_kernel<<<(n + 127) / 128, 128, 0, st>>>(d, s->list, n, s->next_round);
   GPQ_CUDA_TRY(cudaGetLastError());
   GPQ_CUDA_TRY(cudaStreamSynchronize(st));  // the staging buffers are reused
   s->pending.clear();
