@@ -75,9 +75,13 @@ gpq_status astar_normalize(gpq_astar_config& c) {
   GPQ_CHECK_ARG(c.tile_worker <= 1, "tile_worker must be 0 (CTA) or 1 (warp)");
   if (c.frontier_capacity == 0) c.frontier_capacity = c.tile_worker ? 256 : 2048;
   GPQ_CHECK_ARG(c.frontier_capacity >= 64 && c.frontier_capacity <= 8192, "frontier_capacity in [64, 8192]");
-  if (c.block_threads == 0) c.block_threads = 256;
-  GPQ_CHECK_ARG(c.block_threads == 64 || c.block_threads == 128 || c.block_threads == 256,
-                "block_threads must be 64, 128 or 256");
+  if (c.block_threads == 0) {
+    // a thread for 8 cells of a swept tile: 2048 x 2048 search 2.27 ms with 256 threads, 1.97 with 512
+    c.block_threads = c.tile == 64 && !c.tile_worker ? 512 : 256;
+  } else {
+    GPQ_CHECK_ARG(c.block_threads == 64 || c.block_threads == 128 || c.block_threads == 256,
+                  "block_threads must be 64, 128 or 256");
+  }
   if (c.max_rounds == 0) c.max_rounds = 1u << 20;
   return GPQ_OK;
 }
@@ -229,7 +233,7 @@ static gpq_status astar_solve_pass(gpq_astar* a, const gpq_astar_grid* grids, ui
   d.frontier_cap = c.frontier_capacity;
   d.spin_limit = gpq::spin_limit();
   // launch geometry
-  const void* kern = c.tile_worker ? (const void*)astar_persistent_kernel<true> : (const void*)astar_persistent_kernel<false>;
+  const void* kern = astar_kernel(c.tile, c.tile_worker != 0, c.block_threads);
   const size_t smem = astar_worker_smem_bytes(ts, c.frontier_capacity, c.tile_worker, c.block_threads) * (c.tile_worker ? c.block_threads / 32 : 1);
   GPQ_CHECK_ARG(smem <= 227u * 1024u, "tile, frontier_capacity and workers need more than 227 KB of shared memory");
   GPQ_CUDA_TRY(gpq::raise_smem_limit(kern, (int)smem));

@@ -151,7 +151,7 @@ struct AstarTileSmem {
   uint32_t* chg;  // list walk: [ts * ts / 32] cells whose g dropped during this visit
   uint2* ob;      // list walk: [8 * ts] moves into other tiles, sent when the visit ends
   uint16_t* vs;   // sweeps: [ts + 2][astar_sweep_stride] g - g_min of the expanded cells
-  uint32_t flag[2][10];  // sweeps: warps whose cells changed, by parity, a zero at each end
+  uint32_t moved[3];  // sweeps: warps whose cells changed, by barrier mod 3
   uint32_t ob_n;
   uint32_t n[3];  // frontier fill, rotating by level
   uint32_t ub;    // the instance's best goal cost as of this visit (stale values only prune less)
@@ -166,21 +166,22 @@ struct AstarTileSmem {
 
 __host__ __device__ inline uint32_t astar_outbox_cap(uint32_t ts) { return 8u * ts; }
 
-// How a visit walks its tile: a CTA with a thread for 16 cells sweeps tiles of 64 x 64 and
-// 32 x 32 cells (astar_sweep_tile); other tile sides, smaller CTAs, and tiles worked by one
-// warp keep frontier lists (astar_expand_warp).
-__host__ __device__ inline bool astar_sweeps(uint32_t ts, bool warp, uint32_t block) {
-  return !warp && (ts == 64u || ts == 32u) && block >= ts * ts / 16u;
+// How a visit walks its tile: a CTA with a thread for 8 or for 16 cells sweeps tiles of
+// 64 x 64 and 32 x 32 cells (astar_sweep_tile); other tile sides, smaller CTAs, and tiles
+// worked by one warp keep frontier lists (astar_expand_warp).  Returns the pairs of cells
+// a thread holds (4 or 8), or 0 for lists.
+__host__ __device__ inline uint32_t astar_sweep_pairs(uint32_t ts, bool warp, uint32_t block) {
+  if (warp || (ts != 64u && ts != 32u)) return 0;
+  return block >= ts * ts / 8u ? 4u : block >= ts * ts / 16u ? 8u : 0u;
 }
 
 // 16-bit cells of a row in shared memory: 8 in front of the tile's (a 16-byte border, of which
-// the last is the left neighbour), 16 or more behind; rows shift by 12 banks (tiles of 64)
-// so that eight lanes' 16-byte loads from two rows meet 32 different banks.
+// the last is the left neighbour) and 16 behind.
 __host__ __device__ inline uint32_t astar_sweep_stride(uint32_t ts) { return ts + 24u; }
 
 __host__ __device__ inline size_t astar_smem_bytes(uint32_t ts, uint32_t frontier_cap, bool warp, uint32_t block) {
   const size_t cells = (size_t)ts * ts, words = cells / 32;
-  if (astar_sweeps(ts, warp, block))
+  if (astar_sweep_pairs(ts, warp, block))
     return (size_t)(ts + 2u) * astar_sweep_stride(ts) * sizeof(uint16_t) + (size_t)frontier_cap * sizeof(uint2) +
            cells * sizeof(uint32_t) + words * sizeof(uint32_t);
   return 2ull * frontier_cap * sizeof(uint2) + (size_t)astar_outbox_cap(ts) * sizeof(uint2) +
@@ -190,7 +191,7 @@ __host__ __device__ inline size_t astar_smem_bytes(uint32_t ts, uint32_t frontie
 __device__ __forceinline__ void astar_smem_carve(AstarTileSmem& sm, unsigned char* base, uint32_t ts,
                                                  uint32_t frontier_cap, bool warp) {
   const uint32_t words = ts * ts / 32;
-  if (astar_sweeps(ts, warp, blockDim.x)) {
+  if (astar_sweep_pairs(ts, warp, blockDim.x)) {
     sm.vs = reinterpret_cast<uint16_t*>(base);
     sm.gt = reinterpret_cast<uint32_t*>(sm.vs + (ts + 2u) * astar_sweep_stride(ts));
     sm.fa = reinterpret_cast<uint2*>(sm.gt + ts * ts);
@@ -433,8 +434,8 @@ __device__ __forceinline__ uint32_t astar_worker_scan(uint32_t flag, uint32_t* s
 // every wavefront of the tile by one cell in about 250 cycles without lists, atomics or
 // per-cell branches, where a level of a frontier list costs a pass through shared-memory
 // counters and appends.  Warps whose rows and neighbour rows did not change skip a sweep.
-// Measured, search only: 2048 x 2048 4-connected 8.05 -> 2.45 ms, 500 8-connected searches
-// of sides 64 to 1,024 12.0 -> 3.7 ms.
+// Measured, search only, against frontier lists: 2048 x 2048 4-connected 8.05 -> 1.95 ms, 500
+// 8-connected searches of sides 64 to 1,024 12.0 -> 3.2 ms.
 //
 // Only cells that this visit labels, and its items, pass their label on, and only inside
 // the window (label < K): the others' moves were made when they were labelled.  Labels only
@@ -443,8 +444,8 @@ __device__ __forceinline__ uint32_t astar_worker_scan(uint32_t flag, uint32_t* s
 static constexpr uint32_t kSweepInf = 0x7fffu;        // no label
 static constexpr uint32_t kSweepInf2 = 0x7fff7fffu;
 static constexpr uint32_t kSweepSpan = 0x7f00u;       // larger labels are not passed on in this visit
-// Sweeps of a warp between barriers (fewer when its cells stop changing): the 2048 x 2048
-// search takes 3.69 / 3.07 / 2.64 / 2.45 ms with 1 / 2 / 4 / 8.
+// Sweeps of a warp between barriers (fewer when its cells stop changing): with 16 cells a
+// thread the 2048 x 2048 search took 3.69 / 3.07 / 2.64 / 2.45 ms with 1 / 2 / 4 / 8.
 static constexpr uint32_t kSweepsPerBarrier = 8;
 static constexpr uint32_t kSweepMax = 1u << 16;       // sweeps of one visit (at most one per cell is needed)
 
@@ -460,34 +461,52 @@ __device__ __forceinline__ uint32_t astar_pair_below(uint32_t v, uint32_t k1) {
   return v | (~ok & kSweepInf2);
 }
 
-// Pairs shifted by one cell along a row of eight pairs p with neighbours a (left) and b (right).
+// Pairs shifted by one cell along a row of NP pairs p with neighbours a (left) and b (right).
 __device__ __forceinline__ uint32_t astar_pair_left(const uint32_t* p, int i, uint32_t a) {
   return astar_pair_perm(i ? p[i ? i - 1 : 0] : a, p[i], 0x5432u);
 }
+template <int NP>
 __device__ __forceinline__ uint32_t astar_pair_right(const uint32_t* p, int i, uint32_t b) {
-  return astar_pair_perm(p[i], i < 7 ? p[i < 7 ? i + 1 : 7] : b, 0x5432u);
+  return astar_pair_perm(p[i], i < NP - 1 ? p[i < NP - 1 ? i + 1 : 0] : b, 0x5432u);
 }
 
+template <int NP>
 __device__ __forceinline__ void astar_load_row(const uint16_t* row, uint32_t* p, uint32_t& a, uint32_t& b) {
-  const uint4 u = *reinterpret_cast<const uint4*>(row), v = *reinterpret_cast<const uint4*>(row + 8);
-  p[0] = u.x; p[1] = u.y; p[2] = u.z; p[3] = u.w;
-  p[4] = v.x; p[5] = v.y; p[6] = v.z; p[7] = v.w;
+#pragma unroll
+  for (int q = 0; q < NP / 4; ++q) {
+    const uint4 u = *reinterpret_cast<const uint4*>(row + 8 * q);
+    p[4 * q] = u.x;
+    p[4 * q + 1] = u.y;
+    p[4 * q + 2] = u.z;
+    p[4 * q + 3] = u.w;
+  }
   a = *reinterpret_cast<const uint32_t*>(row - 2);
-  b = *reinterpret_cast<const uint32_t*>(row + 16);
+  b = *reinterpret_cast<const uint32_t*>(row + 2 * NP);
 }
 
 // Walks the tile from the n items of sm.fa (all threads; sm.g_min is set, sm.vs all "no
 // label").  On return sm.vs holds the labels of the expanded cells; changed labels are
 // merged into the global g values, labelled cells above the window are in the open array.
-// DIAG: 8-connected, costs 10 and 14; else unit moves.
-template <bool DIAG>
+// DIAG: 8-connected, costs 10 and 14; else unit moves.  NP: pairs of cells of a thread; a
+// warp holds a block of 16 rows x 4 * NP columns, so that a wavefront crossing the tile
+// occupies few of them.
+template <bool DIAG, int NP>
 __device__ __forceinline__ void astar_sweep_tile(const AstarDev& d, AstarInstDev* Ip, const AstarInstDev& I,
                                                  AstarTileSmem& sm, const AstarTileGeo& tg, uint32_t n, uint32_t t,
                                                  uint32_t next_round, uint32_t bound, uint32_t* pops) {
   constexpr uint32_t kStraight = DIAG ? 0x000a000au : 0x00010001u;
   const uint32_t ts = tg.ts, lts = tg.lts, tid = threadIdx.x, stride = astar_sweep_stride(ts);
-  const uint32_t lsegs = lts - 4u, y = tid >> lsegs, xs = (tid & ((1u << lsegs) - 1u)) << 4;
+  const uint32_t warp = tid >> 5, lane = tid & 31u;
+  const uint32_t bcols = ts / (4u * NP), brow = warp / bcols, bcol = warp % bcols;  // the warp's block
+  const uint32_t y = brow * 16u + (lane >> 1), xs = bcol * (4u * NP) + (lane & 1u) * (2u * NP);
   const bool on = y < ts;
+  // blocks whose changes concern this one: itself and its neighbours
+  uint32_t near = 0;
+  for (int i = -1; i <= 1; ++i)
+    for (int j = -1; j <= 1; ++j) {
+      const int r = (int)brow + i, c = (int)bcol + j;
+      if (r >= 0 && c >= 0 && r < (int)(ts / 16u) && c < (int)bcols) near |= 1u << (r * (int)bcols + c);
+    }
   const uint32_t base = sm.g_min, lim = min(bound, sm.ub);
   for (uint32_t i = tid; i < n; i += blockDim.x) {
     const uint2 it = sm.fa[i];
@@ -497,24 +516,25 @@ __device__ __forceinline__ void astar_sweep_tile(const AstarDev& d, AstarInstDev
   }
   __syncthreads();
   uint16_t* row = sm.vs + ((on ? y : 0u) + 1u) * stride + 8u + xs;
-  uint32_t v[8], k1[8];                      // labels; min(old label, window) as astar_pair_below takes it
-  uint32_t cnw[8], cne[8], csw[8], cse[8];   // cost of the diagonal move from each neighbour, 0x8000 = none
-  uint32_t p[8], pa, pb;                     // labels passed on
+  uint32_t v[NP], k1[NP];                        // labels; min(old label, window) as astar_pair_below takes it
+  uint32_t cnw[NP], cne[NP], csw[NP], cse[NP];   // cost of the diagonal move from each neighbour, 0x8000 = none
+  uint32_t p[NP], pa, pb;                        // labels passed on
   uint32_t items = 0;                        // the thread's cells that are items
   const int gx = (int)I.gx - (int)(tg.x0 + xs);
   const uint32_t dyg = (uint32_t)abs((int)(tg.y0 + y) - (int)I.gy);
   if (on) {
-    astar_load_row(row, p, pa, pb);
-    // blocked bits of columns xs - 1 .. xs + 16 of the rows y - 1, y, y + 1 (outside: blocked)
+    astar_load_row<NP>(row, p, pa, pb);
+    // blocked bits of columns xs - 1 .. xs + 2 NP of the rows y - 1, y, y + 1 (outside: blocked)
     uint32_t bu = ~0u, bc = ~0u, bd = ~0u;
     auto bits = [&](uint32_t yy) {
+      constexpr uint32_t n = 2u * NP;
       const uint32_t l = (yy << lts) + xs;
-      uint32_t w = ((sm.blk[l >> 5] >> (l & 31u)) & 0xffffu) << 1;
+      uint32_t w = ((sm.blk[l >> 5] >> (l & 31u)) & ((1u << n) - 1u)) << 1;
       const uint32_t room = tg.tw > xs ? tg.tw - xs : 0u;  // columns inside the grid
-      if (room < 16u) w |= ~0u << (room + 1u);
+      if (room < n) w |= ~0u << (room + 1u);
       w |= (xs == 0u) ? 1u : ((sm.blk[(l - 1u) >> 5] >> ((l - 1u) & 31u)) & 1u);
-      const bool last = xs + 16u >= tg.tw;
-      w |= (last ? 1u : ((sm.blk[(l + 16u) >> 5] >> ((l + 16u) & 31u)) & 1u)) << 17;
+      const bool last = xs + n >= tg.tw;
+      w |= (last ? 1u : ((sm.blk[(l + n) >> 5] >> ((l + n) & 31u)) & 1u)) << (n + 1u);
       return w;
     };
     if (y < tg.th) bc = bits(y);
@@ -523,7 +543,7 @@ __device__ __forceinline__ void astar_sweep_tile(const AstarDev& d, AstarInstDev
       if (y + 1u < tg.th) bd = bits(y + 1u);
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < NP; ++i) {
       uint32_t vv = 0, kk = 0, c0 = 0, c1 = 0, c2 = 0, c3 = 0;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -560,31 +580,30 @@ __device__ __forceinline__ void astar_sweep_tile(const AstarDev& d, AstarInstDev
       p[i] = astar_pair_below(vv, kk);
     }
   }
-  const uint32_t warp = tid >> 5, lane = tid & 31u;
-  const bool warp_on = (warp << 5) < (ts << lsegs);
+  uint32_t moved = ~0u;
   for (uint32_t it = 0;; ++it) {
-    bool any = false;
-    const volatile uint32_t* f = sm.flag[(it + 1u) & 1u] + warp;
-    if (warp_on && (it == 0 || (f[0] | f[1] | f[2]) != 0u)) {
+    if (tid == 0) sm.moved[(it + 1u) % 3u] = 0;  // last read before the barrier before this one
+    if (on && (moved & near)) {  // the same in a whole warp
+      bool any = false;
       for (uint32_t q = 0; q < kSweepsPerBarrier; ++q) {
-        uint32_t up[8], ua, ub2, dn[8], da, db, np[8];
+        uint32_t up[NP], ua, ub2, dn[NP], da, db, np[NP];
         bool changed = false;
-        astar_load_row(row - stride, up, ua, ub2);
-        astar_load_row(row + stride, dn, da, db);
+        astar_load_row<NP>(row - stride, up, ua, ub2);
+        astar_load_row<NP>(row + stride, dn, da, db);
         pa = *reinterpret_cast<const uint32_t*>(row - 2);
-        pb = *reinterpret_cast<const uint32_t*>(row + 16);
+        pb = *reinterpret_cast<const uint32_t*>(row + 2 * NP);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < NP; ++i) {
           uint32_t a = v[i];
           a = __viaddmin_u16x2(astar_pair_left(p, i, pa), kStraight, a);
-          a = __viaddmin_u16x2(astar_pair_right(p, i, pb), kStraight, a);
+          a = __viaddmin_u16x2(astar_pair_right<NP>(p, i, pb), kStraight, a);
           a = __viaddmin_u16x2(up[i], kStraight, a);
           a = __viaddmin_u16x2(dn[i], kStraight, a);
           if (DIAG) {
             a = __viaddmin_u16x2(astar_pair_left(up, i, ua), cnw[i], a);
-            a = __viaddmin_u16x2(astar_pair_right(up, i, ub2), cne[i], a);
+            a = __viaddmin_u16x2(astar_pair_right<NP>(up, i, ub2), cne[i], a);
             a = __viaddmin_u16x2(astar_pair_left(dn, i, da), csw[i], a);
-            a = __viaddmin_u16x2(astar_pair_right(dn, i, db), cse[i], a);
+            a = __viaddmin_u16x2(astar_pair_right<NP>(dn, i, db), cse[i], a);
           }
           changed |= a != v[i];
           v[i] = a;
@@ -592,17 +611,20 @@ __device__ __forceinline__ void astar_sweep_tile(const AstarDev& d, AstarInstDev
         }
         if (changed) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) p[i] = np[i];
-          *reinterpret_cast<uint4*>(row) = make_uint4(p[0], p[1], p[2], p[3]);
-          *reinterpret_cast<uint4*>(row + 8) = make_uint4(p[4], p[5], p[6], p[7]);
+          for (int i = 0; i < NP; ++i) p[i] = np[i];
+#pragma unroll
+          for (int i = 0; i < NP; i += 4)
+            *reinterpret_cast<uint4*>(row + 2 * i) = make_uint4(p[i], p[i + 1], p[i + 2], p[i + 3]);
         }
         const bool w = __any_sync(GPQ_FULL_MASK, changed);
         any |= w;
         if (!w) break;
       }
+      if (any && lane == 0) atomicOr(&sm.moved[it % 3u], 1u << warp);
     }
-    if (lane == 0) sm.flag[it & 1u][warp + 1u] = any ? 1u : 0u;
-    if (!__syncthreads_or(any)) break;
+    __syncthreads();
+    moved = *(volatile uint32_t*)&sm.moved[it % 3u];
+    if (moved == 0u) break;
     if (it == kSweepMax) {
       if (tid == 0) gpq_set_error(&Ip->err, GPQ_ERR_TIMEOUT);
       break;
@@ -612,31 +634,37 @@ __device__ __forceinline__ void astar_sweep_tile(const AstarDev& d, AstarInstDev
   if (on && y < tg.th) {
     uint32_t* G = d.gcost + I.cell0 + (uint64_t)(tg.y0 + y) * I.g.width + tg.x0 + xs;
     const uint32_t ub = sm.ub;
-    uint32_t done = 0;
+    uint32_t passed = 0, fell = 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int x = 0; x < 2 * NP; ++x) {
+      const uint32_t lab = (v[x / 2] >> (16 * (x & 1))) & 0xffffu, g = base + lab;
+      if (((p[x / 2] >> (16 * (x & 1))) & 0xffffu) != kSweepInf) passed |= 1u << x;
+      // no label, and labels that cannot have changed, aside
+      if (lab < kSweepInf && lab != 0u && g < sm.gt[(y << lts) + xs + (uint32_t)x]) fell |= 1u << x;
+    }
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int x = 2 * i + h;
-        const uint32_t lab = (v[i] >> (16 * h)) & 0xffffu, g = base + lab;
-        const bool passed = ((p[i] >> (16 * h)) & 0xffffu) != kSweepInf;
-        done += passed ? 1u : 0u;
-        if (lab >= kSweepInf || lab == 0u) continue;  // no label, or one that cannot have changed
-        if (g >= sm.gt[(y << lts) + xs + (uint32_t)x]) continue;
-        atomicMin(&G[x], g);
-        if (x == gx && dyg == 0u) {
-          atomicMin(&Ip->ub, g);
-          atomicMin(&sm.ub, g);
-        }
-        if (!passed) {
-          const uint2 itm = make_uint2(astar_pack((int)(tg.x0 + xs) + x, (int)(tg.y0 + y)), g);
-          const uint32_t f = g + astar_hxy(I.g.conn, (int)(tg.x0 + xs) + x, (int)(tg.y0 + y), (int)I.gx, (int)I.gy);
-          if (f <= lim) astar_inbox_push(d, Ip, t, next_round, itm);  // beyond the span of this visit's labels
-          else if (f <= ub) astar_open_push(d, Ip, sm, t, itm, f);
-        }
+    for (int x = 0; x < 2 * NP; ++x)
+      if ((fell >> x) & 1u) atomicMin(&G[x], base + ((v[x / 2] >> (16 * (x & 1))) & 0xffffu));
+    if (dyg == 0u && gx >= 0 && gx < 2 * NP && ((fell >> gx) & 1u)) {
+      uint32_t g = 0;
+#pragma unroll
+      for (int x = 0; x < 2 * NP; ++x)
+        if (x == gx) g = base + ((v[x / 2] >> (16 * (x & 1))) & 0xffffu);
+      atomicMin(&Ip->ub, g);
+      atomicMin(&sm.ub, g);
+    }
+    if (fell & ~passed) {
+#pragma unroll
+      for (int x = 0; x < 2 * NP; ++x) {
+        if (!(((fell & ~passed) >> x) & 1u)) continue;
+        const uint32_t g = base + ((v[x / 2] >> (16 * (x & 1))) & 0xffffu);
+        const uint2 itm = make_uint2(astar_pack((int)(tg.x0 + xs) + x, (int)(tg.y0 + y)), g);
+        const uint32_t f = g + astar_hxy(DIAG ? 8 : 4, (int)(tg.x0 + xs) + x, (int)(tg.y0 + y), (int)I.gx, (int)I.gy);
+        if (f <= lim) astar_inbox_push(d, Ip, t, next_round, itm);  // beyond the span of this visit's labels
+        else if (f <= ub) astar_open_push(d, Ip, sm, t, itm, f);
       }
     }
-    *pops += done;
+    *pops += (uint32_t)__popc(passed);
   }
 }
 
@@ -672,19 +700,38 @@ __device__ __forceinline__ void astar_send_border(const AstarDev& d, AstarInstDe
     const int x = (int)(tg.x0 + lx), y = (int)(tg.y0 + ly);
     const uint32_t g = sm.g_min + lab;
     const uint32_t ub = ok ? min(sm.ub, ldcg_u32(&Ip->ub)) : 0u;
+    // blocked bits of the eight (four) neighbours: those in other tiles from memory, all in flight
+    uint32_t word[M], at[M];
+    bool out[M];
+#pragma unroll
+    for (uint32_t k = 0; k < M; ++k) {
+      const int nx = x + gpq_astar_dx((int)k), ny = y + gpq_astar_dy((int)k);
+      const bool grid = ok && nx >= 0 && ny >= 0 && nx < (int)w && ny < (int)h;
+      out[k] = grid && !tg.inside(nx, ny);
+      word[k] = ~0u;  // off the grid: blocked
+      at[k] = 0;
+      if (grid) {
+        const uint32_t c = (uint32_t)ny * w + (uint32_t)nx;
+        const uint64_t b = I.cell0 + c;
+        const uint32_t l = out[k] ? 0u : tg.local(nx, ny);
+        at[k] = out[k] ? (uint32_t)(b & 31u) : l & 31u;
+        word[k] = out[k] ? __ldg(&d.blk[b >> 5]) : sm.blk[l >> 5];
+      }
+    }
+    uint32_t open = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < M; ++k) open |= ((word[k] >> at[k]) & 1u) ? 0u : 1u << k;
     uint32_t old[M];
     bool go[M];
 #pragma unroll
     for (uint32_t k = 0; k < M; ++k) {
-      const int nx = x + gpq_astar_dx((int)k), ny = y + gpq_astar_dy((int)k);
-      go[k] = ok && nx >= 0 && ny >= 0 && nx < (int)w && ny < (int)h && !tg.inside(nx, ny) &&
-              !astar_blocked(d, I, (uint32_t)ny * w + (uint32_t)nx) &&
-              (k < 4 || (!astar_cell_blocked(d, I, sm, tg, nx, y) && !astar_cell_blocked(d, I, sm, tg, x, ny)));
-    }
-#pragma unroll
-    for (uint32_t k = 0; k < M; ++k) {
-      const uint32_t c = (uint32_t)(y + gpq_astar_dy((int)k)) * w + (uint32_t)(x + gpq_astar_dx((int)k));
+      go[k] = out[k] && ((open >> k) & 1u);
+      if (k >= 4) {  // a diagonal: its two straight neighbours (E 0, W 1, S 2, N 3) are free
+        const uint32_t need = (gpq_astar_dx((int)k) > 0 ? 1u : 2u) | (gpq_astar_dy((int)k) > 0 ? 4u : 8u);
+        go[k] = go[k] && (open & need) == need;
+      }
       old[k] = 0;
+      const uint32_t c = (uint32_t)(y + gpq_astar_dy((int)k)) * w + (uint32_t)(x + gpq_astar_dx((int)k));
       if (go[k]) old[k] = atomicMin(&d.gcost[I.cell0 + c], g + gpq_astar_cost(DIAG ? 8 : 4, (int)k));
     }
     uint32_t place[M];  // neighbour tile << 16 | position among the moves into it
@@ -760,7 +807,7 @@ __device__ __forceinline__ void astar_window_step(const AstarDev& d, AstarInstDe
 }
 
 // Process tile t in round s (one worker).
-template <bool WARP>
+template <bool WARP, int NP>
 __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, AstarTileSmem& sm,
                                    const AstarWorker<WARP>& wk) {
   const uint32_t par = s & 1u, next_round = s + 1u;
@@ -805,7 +852,7 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
     atomicAdd(&d.ctl->visits, 1ull);
   }
   // 0. the tile's g values and blocked bits into shared memory
-  const bool sweeps = astar_sweeps(ts, WARP, blockDim.x);
+  constexpr bool sweeps = NP != 0;
   for (uint32_t j = wk.tid; j < words; j += wk.n) {
     sm.blk[j] = 0;
     if (!sweeps) sm.chg[j] = 0;
@@ -814,7 +861,7 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
     uint4* vs4 = reinterpret_cast<uint4*>(sm.vs);
     const uint4 none = make_uint4(kSweepInf2, kSweepInf2, kSweepInf2, kSweepInf2);
     for (uint32_t j = wk.tid; j < (ts + 2u) * astar_sweep_stride(ts) / 8u; j += wk.n) vs4[j] = none;
-    if (wk.tid < 20u) (&sm.flag[0][0])[wk.tid] = 0;
+    if (wk.tid < 3u) sm.moved[wk.tid] = 0;
   }
   // (sixteen loads of a thread in flight at a time: the copy is a round trip to L2 otherwise repeated)
   for (uint32_t l0 = wk.tid; l0 < ts * ts; l0 += 16u * wk.n) {
@@ -898,7 +945,7 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
   }
   // 3. sweeps; the border's moves when all labels stand
   uint32_t pops = 0;
-  if (sweeps) {
+  if constexpr (sweeps) {
     const uint32_t n = min(sm.n[0], d.frontier_cap);
     if (n > 0) {  // the same in every thread
       uint32_t lo = kAstarInf;
@@ -907,10 +954,10 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
       if ((threadIdx.x & 31u) == 0) atomicMin(&sm.g_min, lo);
       wk.sync();
       if (I.g.conn == 4) {
-        astar_sweep_tile<false>(d, Ip, I, sm, tg, n, t, next_round, bound, &pops);
+        astar_sweep_tile<false, NP>(d, Ip, I, sm, tg, n, t, next_round, bound, &pops);
         astar_send_border<false>(d, Ip, I, sm, tg, next_round);
       } else {
-        astar_sweep_tile<true>(d, Ip, I, sm, tg, n, t, next_round, bound, &pops);
+        astar_sweep_tile<true, NP>(d, Ip, I, sm, tg, n, t, next_round, bound, &pops);
         astar_send_border<true>(d, Ip, I, sm, tg, next_round);
       }
     }
@@ -979,8 +1026,11 @@ __host__ __device__ inline size_t astar_worker_smem_bytes(uint32_t ts, uint32_t 
 
 // Rounds s0, s0 + 1, ... until every instance is done, or until `step_rounds` rounds ran
 // (0 = no limit): a resident session resumes at the next round in its next launch.
-template <bool WARP>
-static __global__ void __launch_bounds__(256, 2) astar_persistent_kernel(AstarDev d, uint32_t s0, uint32_t step_rounds) {
+// NP: pairs of cells of a thread that sweeps (astar_sweep_pairs), 0: list walk.  With four
+// pairs one CTA of 512 threads an SM: a second would halve the registers and spill (2048 x
+// 2048 search 1.97 against 2.25 ms, 500 mixed searches 3.16 against 3.29 ms).
+template <bool WARP, int NP>
+static __global__ void __launch_bounds__(NP == 4 ? 512 : 256, NP == 4 ? 1 : 2) astar_persistent_kernel(AstarDev d, uint32_t s0, uint32_t step_rounds) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ AstarTileSmem sms[kAstarMaxWorkers];
   __shared__ uint32_t s_t;
@@ -1005,7 +1055,7 @@ static __global__ void __launch_bounds__(256, 2) astar_persistent_kernel(AstarDe
     }
     // each worker's first tile goes by its number, later ones from a counter
     for (uint32_t j = me; j < n;) {
-      astar_process_tile<WARP>(d, d.al[(size_t)par * d.n_tiles + j], s, sm, wk);
+      astar_process_tile<WARP, NP>(d, d.al[(size_t)par * d.n_tiles + j], s, sm, wk);
       if (n <= workers) break;
       if (WARP) {
         if (wk.tid == 0) j = workers + atomicAdd(&d.ctl->work[cur], 1u);
@@ -1025,6 +1075,16 @@ static __global__ void __launch_bounds__(256, 2) astar_persistent_kernel(AstarDe
       break;
     }
     if (step_rounds && s + 1 - s0 >= step_rounds) break;
+  }
+}
+
+// The kernel for a tile side, worker and CTA size (host side).
+inline const void* astar_kernel(uint32_t ts, bool warp, uint32_t block) {
+  if (warp) return (const void*)astar_persistent_kernel<true, 0>;
+  switch (astar_sweep_pairs(ts, false, block)) {
+    case 4: return (const void*)astar_persistent_kernel<false, 4>;
+    case 8: return (const void*)astar_persistent_kernel<false, 8>;
+    default: return (const void*)astar_persistent_kernel<false, 0>;
   }
 }
 

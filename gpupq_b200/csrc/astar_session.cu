@@ -192,7 +192,7 @@ gpq_status gpq_astar_session_create(const gpq_astar_config* cfg, uint64_t max_ce
     gpq_astar_session_destroy(s);
     return e == cudaErrorMemoryAllocation ? GPQ_ERR_NOMEM : GPQ_ERR_CUDA;
   }
-  s->kern = c.tile_worker ? (const void*)astar_persistent_kernel<true> : (const void*)astar_persistent_kernel<false>;
+  s->kern = astar_kernel(c.tile, c.tile_worker != 0, c.block_threads);
   s->smem = astar_worker_smem_bytes(c.tile, c.frontier_capacity, c.tile_worker, c.block_threads) * (c.tile_worker ? c.block_threads / 32 : 1);
   int dev = 0, sms = 0, per_sm = 0;
   GPQ_CUDA_TRY(gpq::raise_smem_limit(s->kern, (int)s->smem));

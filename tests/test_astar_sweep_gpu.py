@@ -32,8 +32,8 @@ def _grids():
     return np.concatenate(out)
 
 
-@pytest.mark.parametrize("tile,block,worker", [(64, 256, 0), (64, 128, 0), (32, 256, 0), (32, 64, 0), (16, 64, 0),
-                                               (32, 64, 1)])
+@pytest.mark.parametrize("tile,block,worker", [(64, 0, 0), (64, 256, 0), (64, 128, 0), (32, 0, 0), (32, 128, 0),
+                                               (32, 64, 0), (16, 64, 0), (32, 64, 1)])
 @pytest.mark.parametrize("window", [1, 7, 300])
 def test_tile_visit_forms(gpu_lib, tile, block, worker, window):
     grids = _grids()
