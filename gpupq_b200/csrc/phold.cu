@@ -317,12 +317,19 @@ gpq_status gpq_phold_create(const gpq_phold_config* cfg_in, gpq_phold** out) {
   } else if (!phold_kernel_set(c.queue_kind, c.lanes_per_lp, c.insert_capacity, &h->ks, c.laq_mode)) {
     return fail(GPQ_ERR_INVALID);
   }
-  if (!gpq::fit_block_to_smem(&h->block, h->ks.group, h->ks.group_smem + 24 * kStageRounds,
-                              200 * 1024 - 2048 * 16 - 16)) {
+  const size_t block_limit = 200 * 1024 - 2048 * 16 - 16;
+  if (!gpq::fit_block_to_smem(&h->block, h->ks.group, h->ks.group_smem + 24 * kStageRounds, block_limit)) {
     gpq::set_last_error("insert_capacity %u needs too much shared memory per lane group", c.insert_capacity);
     return fail(GPQ_ERR_INVALID);
   }
   h->cfg.block_threads = h->block;
+  const uint32_t lanes = gpq::run_lanes(c, cfg_in->lanes_per_lp);
+  if (!h->is_lab && lanes != c.lanes_per_lp) {  // wider groups: fewer, so they fit too
+    h->block = c.block_threads;
+    if (!phold_kernel_set(c.queue_kind, lanes, c.insert_capacity, &h->ks, c.laq_mode) ||
+        !gpq::fit_block_to_smem(&h->block, h->ks.group, h->ks.group_smem + 24 * kStageRounds, block_limit))
+      return fail(GPQ_ERR_INVALID);
+  }
   const size_t smem = h->window_smem();
   TRY(gpq::raise_smem_limit(h->ks.window, (int)smem));
   TRY(gpq::raise_smem_limit(h->ks.persistent, (int)smem));

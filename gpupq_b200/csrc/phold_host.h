@@ -94,8 +94,31 @@ inline uint32_t lsq_lanes(uint32_t num_lps) {
   return 1;
 }
 
+// Default lanes per LP of the sorted local array queue (laq_mode 0 and 1).  With few LPs a
+// window is one LP's chain of dependent steps, which more lanes shorten, as long as one
+// wave of CTAs holds them all; between one and about three waves of 8-lane groups the last
+// wave is short and 16 lanes even it out; beyond that the CTAs' throughput counts and 8
+// lanes cost least.  Measured (us a window with 8 / 16 / 32 lanes): 1,024 LPs x 16 events
+// 12.2 / 9.0 / 7.5, 2,048 x 16 12.7 / 9.4 / 8.3, 4,096 x 16 13.1 / 10.2 / 11.7, 8,192 x 16
+// 14.7 / 15.5 / 15.4, 20,011 x 32 29.2 / 27.6 / 31.5, 44,133 x 60 66.7 / 65.5 / 71.6,
+// 65,536 x 30 65.9 / 73.6 / 90.2.
+inline uint32_t laq_lanes(uint32_t num_lps) {
+  if (num_lps <= 2048) return 32;
+  if (num_lps <= 4096) return 16;
+  return num_lps > 14208 && num_lps <= 48000 ? 16 : 8;
+}
+
+// Lanes per LP that a run uses: the asked-for number, or by the number of LPs.  `c` is the
+// normalized configuration, which goes into snapshots and keeps 8 (splay queue: 1) for the
+// default, so that a run's state goes between handles whatever their lanes.
+inline uint32_t run_lanes(const gpq_phold_config& c, uint32_t asked) {
+  if (c.queue_kind == GPQ_QUEUE_LSQ) return lsq_lanes(c.num_lps);
+  if (c.queue_kind == GPQ_QUEUE_LAQ && c.laq_mode != 2 && asked == 0) return laq_lanes(c.num_lps);
+  return c.lanes_per_lp;
+}
+
 // Fills the per-kind defaults (capacity 256, insert capacity 64, 256-thread CTAs,
-// 8 lanes per LP; lsq_lanes for the splay queue) and checks them.
+// 8 lanes per LP; one lane for the splay queue) and checks them.
 inline gpq_status normalize_queue_config(gpq_phold_config* c) {
   if (c->capacity == 0) c->capacity = 256;
   if (c->insert_capacity == 0) c->insert_capacity = 64;
@@ -109,7 +132,7 @@ inline gpq_status normalize_queue_config(gpq_phold_config* c) {
   if (c->block_threads == 0) c->block_threads = 256;
   GPQ_CHECK_ARG(c->block_threads % 32 == 0 && c->block_threads >= 32 && c->block_threads <= 1024,
                 "block_threads must be a multiple of 32 in [32, 1024]");
-  if (c->queue_kind == GPQ_QUEUE_LSQ) c->lanes_per_lp = lsq_lanes(c->num_lps);
+  if (c->queue_kind == GPQ_QUEUE_LSQ) c->lanes_per_lp = 1;
   if (c->lanes_per_lp == 0) c->lanes_per_lp = 8;
   if (c->queue_kind == GPQ_QUEUE_LAQ)
     GPQ_CHECK_ARG(c->lanes_per_lp == 4 || c->lanes_per_lp == 8 || c->lanes_per_lp == 16 || c->lanes_per_lp == 32,

@@ -36,3 +36,34 @@ def test_splay_split(gpu_lib, lps, per, la, end):
     for loop in ("persistent", "plain"):
         _check(dict(num_lps=lps, events_per_lp=per, lookahead=la, end_time=end, seed=3, dest_mode=1, ring_width=3),
                "lsq", loop=loop, capacity=512, insert_capacity=512)
+
+
+@pytest.mark.parametrize("lps", [1, 2048, 2049, 4096, 4097, 14208, 14209, 48000, 48001])
+def test_sorted_array_lanes(gpu_lib, lps):
+    for loop in ("persistent", "plain"):
+        _check(dict(num_lps=lps, events_per_lp=9, lookahead=0.4, end_time=4.0, seed=lps, dest_mode=0), "laq", loop=loop)
+
+
+@pytest.mark.parametrize("ibc", [1024, 33])
+def test_sorted_array_insert_capacity(gpu_lib, ibc):
+    """32 lanes per LP with the largest insert buffers (fewer LPs a CTA) and an odd size."""
+    _check(dict(num_lps=300, events_per_lp=20, lookahead=0.3, end_time=6.0, seed=8, dest_mode=1, ring_width=4), "laq",
+           insert_capacity=ibc)
+
+
+@pytest.mark.parametrize("queue", ["laq", "lsq"])
+def test_state_goes_between_lane_counts(gpu_lib, queue):
+    """A run's snapshot fits a handle that asks for the former default lanes, and back."""
+    cfgd = dict(num_lps=900, events_per_lp=12, lookahead=0.5, end_time=12.0, seed=6, dest_mode=0)
+    o = O.phold(O.make_cfg(**cfgd), 8)
+    default = G.make_phold_config(**cfgd, queue=queue)
+    asked = G.make_phold_config(**cfgd, queue=queue, lanes_per_lp=1 if queue == "lsq" else 8)
+    for a, b in ((default, asked), (asked, default)):
+        with G.Phold(a) as x, G.Phold(b) as y:
+            x.populate()
+            x.step(9)
+            y.restore(x.snapshot())
+            y.run()
+            r, s = y.result(), y.lp_stats()
+        assert r["committed"] == o["committed"]
+        assert np.array_equal(s["ohash"], o["ohash"])
