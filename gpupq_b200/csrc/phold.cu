@@ -323,7 +323,8 @@ gpq_status gpq_phold_create(const gpq_phold_config* cfg_in, gpq_phold** out) {
     return fail(GPQ_ERR_INVALID);
   }
   h->cfg.block_threads = h->block;
-  const uint32_t lanes = gpq::run_lanes(c, cfg_in->lanes_per_lp);
+  uint32_t lanes = gpq::run_lanes(c, cfg_in->lanes_per_lp);
+  if (c.queue_kind == GPQ_QUEUE_LHQ && cfg_in->lanes_per_lp == 0 && gpq::lhq_warp(c)) lanes = kLhqWarp;
   if (!h->is_lab && lanes != c.lanes_per_lp) {  // wider groups: fewer, so they fit too
     h->block = c.block_threads;
     if (!phold_kernel_set(c.queue_kind, lanes, c.insert_capacity, &h->ks, c.laq_mode) ||

@@ -108,6 +108,17 @@ inline uint32_t laq_lanes(uint32_t num_lps) {
   return num_lps > 14208 && num_lps <= 48000 ? 16 : 8;
 }
 
+// Whether the local heap queue takes a warp per LP and a window's items in one piece
+// (lhqw_lp_stage) where no number of lanes is asked for: with many events per LP and
+// window, or while one wave of warps holds all LPs; otherwise the warp's fixed steps cost
+// more than a few single pops.  Measured (us a window, 8 lanes / warp; events per LP and
+// window): 1,024 LPs 21.6 / 9.6 (8), 3,000 12.2 / 11.2 (2), 6,000 13.1 / 18.3 (2), 8,191
+// 42.4 / 32.0 (11), 20,011 24.8 / 39.5 (2) and 64.4 / 54.2 (8), 44,123 228 / 130 (20), 65,536
+// 104 / 139 (6) and 117 / 113 (8).
+inline bool lhq_warp(const gpq_phold_config& c) {
+  return c.num_lps <= 4096 || (double)c.events_per_lp * c.lookahead / (1.0 + c.lookahead) >= 7.5;
+}
+
 // Lanes per LP that a run uses: the asked-for number, or by the number of LPs.  `c` is the
 // normalized configuration, which goes into snapshots and keeps 8 (splay queue: 1) for the
 // default, so that a run's state goes between handles whatever their lanes.

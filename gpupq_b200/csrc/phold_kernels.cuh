@@ -34,6 +34,9 @@ template <int G>
 struct LhqP : LhqPolicy<G> {
   __device__ static LhqDev dev(const LpQueueDev& l) { return LhqDev{l.items, l.a, l.cap_log2}; }
 };
+struct LhqWarpP : LhqWarpPolicy {
+  __device__ static LhqDev dev(const LpQueueDev& l) { return LhqDev{l.items, l.a, l.cap_log2}; }
+};
 template <int G>
 struct LsqP : LsqPolicy<G> {
   __device__ static LsqDev dev(const LpQueueDev& l) {
@@ -206,7 +209,8 @@ __device__ __forceinline__ void phold_window_body(const PholdDev& d, const typen
 
 // Plain form: one launch per window; the kernel boundary is the barrier.
 template <class Q>
-static __global__ void phold_window_kernel(PholdDev d, LpQueueDev lq, InsDev ib, uint32_t s) {
+__device__ __forceinline__ void phold_window_launch(const PholdDev& d, const LpQueueDev& lq, const InsDev& ib,
+                                                    uint32_t s) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t red[32];
   const uint32_t mb = d.ctrl->mins[s % 3u];
@@ -225,7 +229,8 @@ static __global__ void phold_window_kernel(PholdDev d, LpQueueDev lq, InsDev ib,
 // separates windows.  Every block takes the same exit decision from the same
 // (minimum, error) slot written before the barrier.
 template <class Q>
-static __global__ void phold_persistent_kernel(PholdDev d, LpQueueDev lq, InsDev ib, uint32_t s0, uint32_t max_steps) {
+__device__ __forceinline__ void phold_persistent_launch(const PholdDev& d, const LpQueueDev& lq, const InsDev& ib,
+                                                        uint32_t s0, uint32_t max_steps) {
   const typename Q::Dev q = Q::dev(lq);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t red[32];
@@ -251,6 +256,25 @@ static __global__ void phold_persistent_kernel(PholdDev d, LpQueueDev lq, InsDev
   if (blockIdx.x == 0 && threadIdx.x == 0) d.ctrl->phase = s;
 }
 
+template <class Q>
+static __global__ void phold_window_kernel(PholdDev d, LpQueueDev lq, InsDev ib, uint32_t s) {
+  phold_window_launch<Q>(d, lq, ib, s);
+}
+template <class Q>
+static __global__ void phold_persistent_kernel(PholdDev d, LpQueueDev lq, InsDev ib, uint32_t s0, uint32_t max_steps) {
+  phold_persistent_launch<Q>(d, lq, ib, s0, max_steps);
+}
+// At most 64 registers a thread: CTAs of up to 1,024 threads fit.
+template <class Q>
+static __global__ void __launch_bounds__(1024) phold_window_kernel64(PholdDev d, LpQueueDev lq, InsDev ib, uint32_t s) {
+  phold_window_launch<Q>(d, lq, ib, s);
+}
+template <class Q>
+static __global__ void __launch_bounds__(1024) phold_persistent_kernel64(PholdDev d, LpQueueDev lq, InsDev ib,
+                                                                         uint32_t s0, uint32_t max_steps) {
+  phold_persistent_launch<Q>(d, lq, ib, s0, max_steps);
+}
+
 // Kernel pointers of one (queue kind, lane-group size) pair (host-side dispatch).
 struct PholdKernelSet {
   const void* window;
@@ -259,9 +283,14 @@ struct PholdKernelSet {
   size_t group_smem;  // per lane group, for insert capacity ibc
 };
 
+// group kLhqWarp: the local heap queue's form of a warp per LP.
+static constexpr uint32_t kLhqWarp = 132;
+
 inline bool phold_kernel_set(uint32_t kind, uint32_t group, uint32_t ibc, PholdKernelSet* out, uint32_t laq_mode = 0) {
 #define GPQ_KS(P) *out = {(const void*)phold_window_kernel<P>, (const void*)phold_persistent_kernel<P>, \
                           (uint32_t)P::G, P::group_smem_bytes(ibc)}; return true
+#define GPQ_KS64(P) *out = {(const void*)phold_window_kernel64<P>, (const void*)phold_persistent_kernel64<P>, \
+                            (uint32_t)P::G, P::group_smem_bytes(ibc)}; return true
   if (kind == GPQ_QUEUE_LAQ && laq_mode == 1) {
     switch (group) {
       case 4: GPQ_KS(LasP<4>);
@@ -278,6 +307,7 @@ inline bool phold_kernel_set(uint32_t kind, uint32_t group, uint32_t ibc, PholdK
     }
   } else if (kind == GPQ_QUEUE_LHQ) {
     switch (group) {
+      case kLhqWarp: GPQ_KS64(LhqWarpP);
       case 1: GPQ_KS(LhqP<1>);
       case 4: GPQ_KS(LhqP<4>);
       case 8: GPQ_KS(LhqP<8>);
@@ -286,14 +316,15 @@ inline bool phold_kernel_set(uint32_t kind, uint32_t group, uint32_t ibc, PholdK
     }
   } else if (kind == GPQ_QUEUE_LSQ) {
     switch (group) {
-      case 1: GPQ_KS(LsqP<1>);
-      case 4: GPQ_KS(LsqP<4>);
-      case 8: GPQ_KS(LsqP<8>);
-      case 16: GPQ_KS(LsqP<16>);
-      case 32: GPQ_KS(LsqP<32>);
+      case 1: GPQ_KS64(LsqP<1>);
+      case 4: GPQ_KS64(LsqP<4>);
+      case 8: GPQ_KS64(LsqP<8>);
+      case 16: GPQ_KS64(LsqP<16>);
+      case 32: GPQ_KS64(LsqP<32>);
     }
   }
 #undef GPQ_KS
+#undef GPQ_KS64
   return false;
 }
 

@@ -44,6 +44,26 @@ def test_sorted_array_lanes(gpu_lib, lps):
         _check(dict(num_lps=lps, events_per_lp=9, lookahead=0.4, end_time=4.0, seed=lps, dest_mode=0), "laq", loop=loop)
 
 
+@pytest.mark.parametrize("lps,per,la,end,ring", [
+    (1, 1, 0.5, 30.0, 0), (40, 1, 0.01, 3.0, 1), (4096, 9, 0.4, 6.0, 0), (4097, 9, 0.4, 6.0, 0), (4500, 17, 0.8, 8.0, 0),
+    (300, 9, 3.0, 30.0, 1),     # most of a heap safe in every window
+    (200, 73, 0.3, 6.0, 1), (200, 74, 0.02, 1.0, 1), (150, 600, 0.01, 0.4, 1),  # full levels, one more, four levels
+    (200, 150, 20.0, 60.0, 1),  # more safe items than the warp form takes: event by event
+])
+def test_local_heap_windows(gpu_lib, lps, per, la, end, ring):
+    for loop in ("persistent", "plain"):
+        _check(dict(num_lps=lps, events_per_lp=per, lookahead=la, end_time=end, seed=per + lps, dest_mode=ring,
+                    ring_width=3), "lhq", loop=loop, capacity=2048 if per > 256 else 512, insert_capacity=512)
+
+
+@pytest.mark.parametrize("queue", ["lhq", "lsq"])
+def test_largest_ctas(gpu_lib, queue):
+    """CTAs of 1,024 threads, which the register use has to allow."""
+    for loop in ("persistent", "plain"):
+        _check(dict(num_lps=900, events_per_lp=9, lookahead=0.4, end_time=4.0, seed=4, dest_mode=0), queue, loop=loop,
+               block_threads=1024)
+
+
 @pytest.mark.parametrize("ibc", [1024, 33])
 def test_sorted_array_insert_capacity(gpu_lib, ibc):
     """32 lanes per LP with the largest insert buffers (fewer LPs a CTA) and an odd size."""
@@ -51,7 +71,7 @@ def test_sorted_array_insert_capacity(gpu_lib, ibc):
            insert_capacity=ibc)
 
 
-@pytest.mark.parametrize("queue", ["laq", "lsq"])
+@pytest.mark.parametrize("queue", ["laq", "lsq", "lhq"])
 def test_state_goes_between_lane_counts(gpu_lib, queue):
     """A run's snapshot fits a handle that asks for the former default lanes, and back."""
     cfgd = dict(num_lps=900, events_per_lp=12, lookahead=0.5, end_time=12.0, seed=6, dest_mode=0)
