@@ -229,6 +229,14 @@ def _ptr(a):
     return ctypes.c_void_p(a.ctypes.data) if a is not None else None
 
 
+def _first(items, n):
+    """The first n items: of the array itself when they are at least half of it, else as a
+    copy, made from bytes (numpy copies an array of records field by field)."""
+    if 2 * n >= len(items):
+        return items[:n]
+    return items.view(np.uint8)[: n * ITEM_DTYPE.itemsize].copy().view(ITEM_DTYPE)
+
+
 def ring_threshold(frac: float) -> int:
     """Probability -> 32-bit threshold floor(frac * 2^32), computed in double."""
     return min(int(frac * 4294967296.0), 0xFFFFFFFF)
@@ -431,11 +439,11 @@ class Queue:
 
     def dequeue(self, bound, max_per_lp=0, capacity=None):
         cap = capacity if capacity is not None else 1 << 20
-        out = np.zeros(cap, ITEM_DTYPE)
+        out = np.empty(cap, ITEM_DTYPE)
         n = ctypes.c_uint64()
         check(lib().gpq_queue_dequeue(self._h, bound, max_per_lp, _ptr(out), cap, ctypes.byref(n), None),
               "gpq_queue_dequeue")
-        return out[: n.value].copy()
+        return _first(out, n.value)
 
     def length(self, lp):
         v = ctypes.c_uint32()
@@ -449,7 +457,7 @@ class Queue:
         out = np.zeros(capacity, ITEM_DTYPE)
         n = ctypes.c_uint64()
         check(lib().gpq_queue_dump(self._h, lp, _ptr(out), capacity, ctypes.byref(n), None), "gpq_queue_dump")
-        return out[: n.value].copy()
+        return _first(out, n.value)
 
     def counts(self):
         a, b = ctypes.c_uint64(), ctypes.c_uint64()
