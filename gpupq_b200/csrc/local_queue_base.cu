@@ -1,5 +1,6 @@
 // Shared plumbing of the per-LP queue objects, and the queue-kind factory.
 #include <algorithm>
+#include <cstring>
 
 #include "local_queue_base.h"
 
@@ -55,7 +56,7 @@ LocalQueueBase::~LocalQueueBase() {
   for (void* p : {(void*)ibuf_, (void*)icnt_, (void*)ctr_, (void*)staging_, (void*)dq_cnt_, (void*)dq_off_,
                   (void*)dq_out_})
     if (p) cudaFree(p);
-  if (h_ctr_) cudaFreeHost(h_ctr_);
+  if (h_) cudaFreeHost(h_);
   if (own_) cudaStreamDestroy(own_);
 }
 
@@ -66,7 +67,7 @@ gpq_status LocalQueueBase::init_base(uint32_t L, uint32_t ibc) {
   GPQ_CUDA_TRY(cudaMalloc(&ibuf_, (size_t)L * ibc * sizeof(gpq_item)));
   GPQ_CUDA_TRY(cudaMalloc(&icnt_, (size_t)L * sizeof(uint32_t)));
   GPQ_CUDA_TRY(cudaMalloc(&ctr_, sizeof(LocalQueueCounters)));
-  GPQ_CUDA_TRY(cudaMallocHost(&h_ctr_, sizeof(LocalQueueCounters)));
+  GPQ_CUDA_TRY(cudaMallocHost(&h_, sizeof(LocalQueueHost)));
   GPQ_CUDA_TRY(cudaMalloc(&dq_cnt_, (size_t)L * sizeof(uint32_t)));
   GPQ_CUDA_TRY(cudaMalloc(&dq_off_, (size_t)(L + 1) * sizeof(unsigned long long)));
   GPQ_CUDA_TRY(cudaMemsetAsync(icnt_, 0, (size_t)L * sizeof(uint32_t), own_));
@@ -77,7 +78,10 @@ gpq_status LocalQueueBase::init_base(uint32_t L, uint32_t ibc) {
 
 gpq_status LocalQueueBase::insert(const gpq_item* items, uint64_t n, bool on_device, cudaStream_t st) {
   const gpq_item* src = items;
-  if (!on_device) {
+  if (!on_device && n <= kHostStageItems) {  // read by the kernel where it is
+    std::memcpy(h_->stage, items, n * sizeof(gpq_item));
+    src = h_->stage;
+  } else if (!on_device) {
     if (staging_n_ < n) {
       if (staging_) cudaFree(staging_);
       staging_ = nullptr;
@@ -96,17 +100,17 @@ gpq_status LocalQueueBase::insert(const gpq_item* items, uint64_t n, bool on_dev
 }
 
 gpq_status LocalQueueBase::counts(uint64_t* enqueued, uint64_t* dequeued, cudaStream_t st) {
-  GPQ_CUDA_TRY(cudaMemcpyAsync(h_ctr_, ctr_, sizeof(LocalQueueCounters), cudaMemcpyDeviceToHost, st));
+  GPQ_CUDA_TRY(cudaMemcpyAsync(&h_->ctr, ctr_, sizeof(LocalQueueCounters), cudaMemcpyDeviceToHost, st));
   GPQ_CUDA_TRY(cudaStreamSynchronize(st));
-  *enqueued = h_ctr_->enqueued;
-  *dequeued = h_ctr_->dequeued;
+  *enqueued = h_->ctr.enqueued;
+  *dequeued = h_->ctr.dequeued;
   return GPQ_OK;
 }
 
 gpq_status LocalQueueBase::take_error(cudaStream_t st) {
-  GPQ_CUDA_TRY(cudaMemcpyAsync(&h_ctr_->err, &ctr_->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  GPQ_CUDA_TRY(cudaMemcpyAsync(&h_->ctr.err, &ctr_->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   GPQ_CUDA_TRY(cudaStreamSynchronize(st));
-  const uint32_t e = h_ctr_->err;
+  const uint32_t e = h_->ctr.err;
   if (e) {
     GPQ_CUDA_TRY(cudaMemsetAsync(&ctr_->err, 0, sizeof(uint32_t), st));
     set_last_error("queue operation reported status %u", e);

@@ -18,7 +18,34 @@ struct LocalQueueCounters {
   unsigned long long dequeued;
   uint32_t err;
   uint32_t min_bits;
+  uint32_t done;  // CTAs of the running kernel that are through (reset by the last)
+  uint32_t pad;
 };
+
+// Page-locked host block that kernels read and write in place: a copy of a few bytes or
+// kilobytes by the copy engine costs more than the kernel it belongs to.
+constexpr uint32_t kHostStageItems = 8192;
+struct LocalQueueHost {
+  LocalQueueCounters ctr;        // copies of the device counters
+  unsigned long long total;      // items of a dequeue
+  uint32_t err, min_bits;        // published by the last CTA of a kernel
+  gpq_item stage[kHostStageItems];  // items of small inserts and dequeues
+};
+
+// True in every thread of the last CTA to call it in this launch; everything the CTAs wrote
+// before is visible to it.
+__device__ __forceinline__ bool lq_last_cta(LocalQueueCounters* ctr) {
+  __shared__ uint32_t s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(&ctr->done, 1u) == gridDim.x - 1u ? 1u : 0u;
+    if (s_last) ctr->done = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  return s_last != 0u;
+}
 
 // queue_insert for a batch (src/local_array_queue.cu:486-513): reserve a slot in the
 // item's LP buffer with atomicAdd; a full buffer records GPQ_ERR_INSERT_FULL.
@@ -49,7 +76,7 @@ class LocalQueueBase : public QueueImpl {
   gpq_item* ibuf_ = nullptr;  // [L][ibc]
   uint32_t* icnt_ = nullptr;  // [L]
   LocalQueueCounters* ctr_ = nullptr;
-  LocalQueueCounters* h_ctr_ = nullptr;  // pinned
+  LocalQueueHost* h_ = nullptr;  // page-locked
   gpq_item* staging_ = nullptr;
   uint64_t staging_n_ = 0;
   uint32_t* dq_cnt_ = nullptr;             // [L] per-LP dequeue counts

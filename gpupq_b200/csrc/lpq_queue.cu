@@ -241,9 +241,9 @@ class LpqQueue final : public LocalQueueBase {
     GPQ_CUDA_TRY(cudaMemcpyAsync(&ctr_->min_bits, &inf, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
     lpq_min_kernel<<<grid(), 256, 0, st>>>(d_, L_, ctr_);
     GPQ_CUDA_TRY(cudaGetLastError());
-    GPQ_CUDA_TRY(cudaMemcpyAsync(&h_ctr_->min_bits, &ctr_->min_bits, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    GPQ_CUDA_TRY(cudaMemcpyAsync(&h_->ctr.min_bits, &ctr_->min_bits, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     GPQ_CUDA_TRY(cudaStreamSynchronize(st));
-    *min_ts = gpq_u2f(h_ctr_->min_bits);
+    *min_ts = gpq_u2f(h_->ctr.min_bits);
     return GPQ_OK;
   }
 
