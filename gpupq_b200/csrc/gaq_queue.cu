@@ -4,6 +4,7 @@
 // max_per_lp items below the bound (the reference's mark_safe_events takes one per LP,
 // :147-179) and compacts the rest back in order.
 #include <algorithm>
+#include <cstring>
 #include <new>
 #include <vector>
 
@@ -16,6 +17,96 @@ namespace gpq {
 
 namespace {
 
+// ---- dequeue without a limit per LP: the array's whole prefix below the bound ----
+// The prefix leaves by moving the array's start, so nothing is compacted; its items are
+// listed per LP (positions, any order), a CTA of 256 threads takes 32 LPs, adds up the
+// counts in front of its own, ranks its LPs' items by key in shared memory and writes them
+// in (LP, key) order.
+constexpr uint32_t kEmitLps = 32;
+constexpr uint32_t kEmitKeys = 2048;  // items of a CTA ranked in shared memory, more from the array
+constexpr uint32_t kEmitCtas = 8192;
+constexpr uint32_t kHostStageItems = 8192;  // items written straight into page-locked memory
+
+// prefix[0] = number of items below the bound.
+__global__ void gq_list_kernel(const gpq_item* __restrict__ arr, const uint32_t* prefix, uint32_t L, uint32_t* idx,
+                               uint32_t* cnt, uint32_t ibc, uint32_t* err) {
+  const uint32_t c = prefix[0];
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < c; i += gridDim.x * blockDim.x) {
+    const uint32_t lp = arr[i].lp;
+    if (lp >= L) { gpq_set_error(err, GPQ_ERR_INVALID); continue; }
+    const uint32_t slot = atomicAdd(&cnt[lp], 1u);
+    if (slot < ibc) idx[(size_t)lp * ibc + slot] = i;
+    else gpq_set_error(err, GPQ_ERR_INSERT_FULL);
+  }
+}
+
+// Sums of 32 LPs' counts, one warp each.
+__global__ void gq_sum_kernel(const uint32_t* __restrict__ cnt, uint32_t L, uint32_t* sums, uint32_t n) {
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lp = w * kEmitLps + (threadIdx.x & 31u);
+  if (w >= n) return;
+  const uint32_t s = warp_sum_u32(lp < L ? cnt[lp] : 0u);
+  if ((threadIdx.x & 31u) == 0) sums[w] = s;
+}
+
+__global__ void __launch_bounds__(256) gq_emit_kernel(const gpq_item* __restrict__ arr, uint32_t L,
+                                                      const uint32_t* __restrict__ idx, uint32_t* cnt, uint32_t ibc,
+                                                      const uint32_t* __restrict__ sums, gpq_item* out) {
+  __shared__ uint64_t s_key[kEmitKeys];
+  __shared__ uint32_t s_off[kEmitLps + 1], s_red[8];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t before = 0;
+  for (uint32_t i = threadIdx.x; i < blockIdx.x; i += blockDim.x) before += sums[i];
+  before = warp_sum_u32(before);
+  if (lane == 0) s_red[warp] = before;
+  if (warp == 0) {
+    const uint32_t lp = blockIdx.x * kEmitLps + lane;
+    const uint32_t c = lp < L ? cnt[lp] : 0u;
+    uint32_t incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(GPQ_FULL_MASK, incl, o);
+      if (lane >= (uint32_t)o) incl += u;
+    }
+    s_off[lane] = incl - c;
+    if (lane == 31u) s_off[32] = incl;
+    if (c) cnt[lp] = 0;  // empty lists for the next dequeue
+  }
+  __syncthreads();
+  before = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) before += s_red[w];
+  const uint32_t n = s_off[kEmitLps];
+  const bool keys = n <= kEmitKeys;
+  auto lp_of = [&](uint32_t j) {  // the last LP whose items start at or before j
+    uint32_t a = 0, b = kEmitLps;
+    while (b - a > 1u) {
+      const uint32_t m = (a + b) >> 1;
+      if (s_off[m] <= j) a = m; else b = m;
+    }
+    return a;
+  };
+  auto place = [&](uint32_t a, uint32_t i) { return idx[(size_t)(blockIdx.x * kEmitLps + a) * ibc + i]; };
+  if (keys) {
+    for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
+      const uint32_t a = lp_of(j);
+      s_key[j] = gpq_lp_key(arr[place(a, j - s_off[a])]);
+    }
+    __syncthreads();
+  }
+  for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
+    const uint32_t a = lp_of(j), j0 = s_off[a], k = s_off[a + 1u] - j0;
+    const gpq_item e = arr[place(a, j - j0)];
+    const uint64_t ke = gpq_lp_key(e);
+    uint32_t r = 0;
+    for (uint32_t i = 0; i < k; ++i) {
+      const uint64_t o = keys ? s_key[j0 + i] : gpq_lp_key(arr[place(a, i)]);
+      r += (o < ke || (o == ke && j0 + i < j)) ? 1u : 0u;
+    }
+    out[before + j0 + r] = e;
+  }
+}
+
+// ---- dequeue with a limit per LP: what stays of the prefix is compacted ----
 // Staged index lists per LP: idx[lp * ibc + slot] = array position.
 __global__ void gq_stage_idx_kernel(const gpq_item* __restrict__ arr, uint32_t c, uint32_t L, uint32_t* idx,
                                     uint32_t* cnt, uint32_t ibc, uint32_t* err) {
@@ -112,9 +203,9 @@ class GaqQueue final : public QueueImpl {
   ~GaqQueue() override {
     for (void* p : {(void*)arr_[0], (void*)arr_[1], (void*)pend_, (void*)pend_tmp_, (void*)hist_, (void*)scan_tmp_, (void*)idx_,
                     (void*)cnt_, (void*)out_cnt_, (void*)off_, (void*)tmp_, (void*)taken_, (void*)keep_,
-                    (void*)words_, (void*)out_, (void*)split_})
+                    (void*)words_, (void*)out_, (void*)split_, (void*)sums_})
       if (p) cudaFree(p);
-    if (h_words_) cudaFreeHost(h_words_);
+    if (h_) cudaFreeHost(h_);
     if (own_) cudaStreamDestroy(own_);
   }
 
@@ -143,7 +234,9 @@ class GaqQueue final : public QueueImpl {
     GPQ_CUDA_TRY(cudaMalloc(&taken_, (size_t)(cap_ + 1) * sizeof(uint32_t)));
     GPQ_CUDA_TRY(cudaMalloc(&keep_, (size_t)(cap_ + 1) * sizeof(uint32_t)));
     GPQ_CUDA_TRY(cudaMalloc(&words_, 16 * sizeof(uint32_t)));
-    GPQ_CUDA_TRY(cudaMallocHost(&h_words_, 16 * sizeof(uint32_t)));
+    GPQ_CUDA_TRY(cudaMalloc(&sums_, (size_t)emit_ctas() * sizeof(uint32_t)));
+    GPQ_CUDA_TRY(cudaMallocHost(&h_, sizeof(Host)));
+    h_words_ = h_->words;
     GPQ_CUDA_TRY(cudaMemsetAsync(cnt_, 0, (size_t)L_ * sizeof(uint32_t), own_));
     GPQ_CUDA_TRY(cudaMemsetAsync(words_, 0, 16 * sizeof(uint32_t), own_));
     GPQ_CUDA_TRY(cudaStreamSynchronize(own_));
@@ -181,9 +274,10 @@ class GaqQueue final : public QueueImpl {
     gpq_status s = radix_sort_by_ts(pend_, pend_tmp_, npend_, h_words_[0], h_words_[1], hist_, &sorted,
                                     words_ + kBulkErrWord, st);
     if (s != GPQ_OK) return s;
-    s = merge_by_ts(arr_[cur_], n_, sorted, npend_, arr_[cur_ ^ 1], split_, words_ + kBulkErrWord, st);
+    s = merge_by_ts(base(), n_, sorted, npend_, arr_[cur_ ^ 1], split_, words_ + kBulkErrWord, st);
     if (s != GPQ_OK) return s;
     cur_ ^= 1;
+    head_ = 0;
     n_ += npend_;
     npend_ = 0;
     uint32_t berr = 0;
@@ -199,7 +293,7 @@ class GaqQueue final : public QueueImpl {
   gpq_status get_min(float* min_ts, cudaStream_t st) override {
     uint32_t b = kInfBits;
     if (n_) {
-      GPQ_CUDA_TRY(cudaMemcpyAsync(&b, &arr_[cur_][0].ts, 4, cudaMemcpyDeviceToHost, st));
+      GPQ_CUDA_TRY(cudaMemcpyAsync(&b, &base()->ts, 4, cudaMemcpyDeviceToHost, st));
       GPQ_CUDA_TRY(cudaStreamSynchronize(st));
     }
     *min_ts = gpq_u2f(b);
@@ -210,7 +304,8 @@ class GaqQueue final : public QueueImpl {
                      cudaStream_t st) override {
     *n_out = 0;
     if (n_ == 0) return GPQ_OK;
-    const gpq_item* a = arr_[cur_];
+    if (max_per_lp == 0 && emit_ctas() <= kEmitCtas) return dequeue_prefix(bound, out, out_capacity, n_out, st);
+    const gpq_item* a = base();
     gaq_split_kernel<<<1, 32, 0, st>>>(a, n_, bound, 3.0e38f, words_);
     GPQ_CUDA_TRY(cudaMemcpyAsync(h_words_, words_, 4, cudaMemcpyDeviceToHost, st));
     GPQ_CUDA_TRY(cudaStreamSynchronize(st));
@@ -248,14 +343,52 @@ class GaqQueue final : public QueueImpl {
     if (total) GPQ_CUDA_TRY(cudaMemcpyAsync(out, out_, (size_t)total * sizeof(gpq_item), cudaMemcpyDeviceToHost, st));
     GPQ_CUDA_TRY(cudaStreamSynchronize(st));
     cur_ ^= 1;
+    head_ = 0;
     n_ -= total;
     deq_ += total;
     return GPQ_OK;
   }
 
+  gpq_status dequeue_prefix(float bound, gpq_item* out, uint64_t out_capacity, uint64_t* n_out, cudaStream_t st) {
+    const gpq_item* a = base();
+    const uint32_t ctas = emit_ctas();
+    GPQ_CUDA_TRY(cudaMemsetAsync(&words_[8], 0, 4, st));
+    gaq_split_kernel<<<1, 32, 0, st>>>(a, n_, bound, 3.0e38f, words_);
+    gq_list_kernel<<<grid(n_), 256, 0, st>>>(a, words_, L_, idx_, cnt_, lpcap_, &words_[8]);
+    gq_sum_kernel<<<(ctas + 7) / 8, 256, 0, st>>>(cnt_, L_, sums_, ctas);
+    GPQ_CUDA_TRY(cudaGetLastError());
+    GPQ_CUDA_TRY(cudaMemcpyAsync(h_words_, words_, 9 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    GPQ_CUDA_TRY(cudaStreamSynchronize(st));
+    const uint32_t c = h_words_[0], e = h_words_[8];
+    if (!e) *n_out = c;
+    if (e || c > out_capacity) {
+      GPQ_CUDA_TRY(cudaMemsetAsync(cnt_, 0, (size_t)L_ * sizeof(uint32_t), st));
+      if (e) return (gpq_status)e;
+      set_last_error("dequeue: %u items do not fit the output", c);
+      return GPQ_ERR_INVALID;
+    }
+    if (c == 0) return GPQ_OK;
+    const bool stage = c <= kHostStageItems;
+    if (!stage && (!out_ || out_n_ < c)) {
+      if (out_) cudaFree(out_);
+      out_ = nullptr;
+      GPQ_CUDA_TRY(cudaMalloc(&out_, (size_t)c * sizeof(gpq_item)));
+      out_n_ = c;
+    }
+    gq_emit_kernel<<<ctas, 256, 0, st>>>(a, L_, idx_, cnt_, lpcap_, sums_, stage ? h_->stage : out_);
+    GPQ_CUDA_TRY(cudaGetLastError());
+    if (!stage) GPQ_CUDA_TRY(cudaMemcpyAsync(out, out_, (size_t)c * sizeof(gpq_item), cudaMemcpyDeviceToHost, st));
+    GPQ_CUDA_TRY(cudaStreamSynchronize(st));
+    if (stage) std::memcpy(out, h_->stage, (size_t)c * sizeof(gpq_item));
+    n_ -= c;
+    head_ = n_ ? head_ + c : 0;
+    deq_ += c;
+    return GPQ_OK;
+  }
+
   gpq_status length(uint32_t lp, uint32_t* len, cudaStream_t st) override {
     GPQ_CUDA_TRY(cudaMemsetAsync(&words_[9], 0, 4, st));
-    if (n_) gq_count_lp_kernel<<<grid(n_), 256, 0, st>>>(arr_[cur_], n_, lp, &words_[9]);
+    if (n_) gq_count_lp_kernel<<<grid(n_), 256, 0, st>>>(base(), n_, lp, &words_[9]);
     GPQ_CUDA_TRY(cudaMemcpyAsync(len, &words_[9], 4, cudaMemcpyDeviceToHost, st));
     GPQ_CUDA_TRY(cudaStreamSynchronize(st));
     return GPQ_OK;
@@ -263,10 +396,10 @@ class GaqQueue final : public QueueImpl {
 
   gpq_status clear(uint32_t lp, cudaStream_t st) override {
     if (n_ == 0) return GPQ_OK;
-    gq_clear_lp_kernel<<<grid(n_ + 1), 256, 0, st>>>(arr_[cur_], n_, lp, keep_);
+    gq_clear_lp_kernel<<<grid(n_ + 1), 256, 0, st>>>(base(), n_, lp, keep_);
     GPQ_CUDA_TRY(cudaMemcpyAsync(taken_, keep_, (size_t)(n_ + 1) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
     if (gpq_status s_ = scan_exclusive(keep_, keep_, n_ + 1, scan_tmp_, st)) return s_;
-    gq_select_kernel<<<grid(n_), 256, 0, st>>>(arr_[cur_], n_, taken_, keep_, arr_[cur_ ^ 1]);
+    gq_select_kernel<<<grid(n_), 256, 0, st>>>(base(), n_, taken_, keep_, arr_[cur_ ^ 1]);
     GPQ_CUDA_TRY(cudaGetLastError());
     uint32_t kept = 0;
     GPQ_CUDA_TRY(cudaMemcpyAsync(&kept, keep_ + n_, 4, cudaMemcpyDeviceToHost, st));
@@ -274,6 +407,7 @@ class GaqQueue final : public QueueImpl {
     deq_ += n_ - kept;
     n_ = kept;
     cur_ ^= 1;
+    head_ = 0;
     return GPQ_OK;
   }
 
@@ -281,7 +415,7 @@ class GaqQueue final : public QueueImpl {
   // of equal timestamps are done on a host copy).
   gpq_status dump(uint32_t lp, gpq_item* out, uint64_t out_capacity, uint64_t* n_out, cudaStream_t st) override {
     std::vector<gpq_item> h(n_);
-    if (n_) GPQ_CUDA_TRY(cudaMemcpyAsync(h.data(), arr_[cur_], (size_t)n_ * sizeof(gpq_item), cudaMemcpyDeviceToHost, st));
+    if (n_) GPQ_CUDA_TRY(cudaMemcpyAsync(h.data(), base(), (size_t)n_ * sizeof(gpq_item), cudaMemcpyDeviceToHost, st));
     GPQ_CUDA_TRY(cudaStreamSynchronize(st));
     std::vector<gpq_item> sel;
     for (const gpq_item& e : h)
@@ -305,6 +439,15 @@ class GaqQueue final : public QueueImpl {
   cudaStream_t own_ = nullptr;
   gpq_item* arr_[2] = {nullptr, nullptr};
   int cur_ = 0;
+  uint32_t head_ = 0;  // the array's items are arr_[cur_][head_, head_ + n_)
+  const gpq_item* base() const { return arr_[cur_] + head_; }
+  uint32_t emit_ctas() const { return (L_ + kEmitLps - 1) / kEmitLps; }
+  uint32_t* sums_ = nullptr;  // [emit_ctas()]
+  struct Host {               // page-locked
+    uint32_t words[16];
+    gpq_item stage[kHostStageItems];
+  };
+  Host* h_ = nullptr;
   uint32_t n_ = 0, npend_ = 0;
   uint64_t enq_ = 0, deq_ = 0;
   gpq_item* pend_ = nullptr;
