@@ -24,6 +24,12 @@
 //   * when the root holds every item (the global array queue's layout; the reference's
 //     256 K root on small populations), a window is three phases over bucket lists that
 //     each phase fills for the next, instead of grid-wide sorts (see the list section).
+// What bounds that form: at 1,024 LPs x 16 the phases' chains of block steps and three
+// barriers (21 us a window of 8,200 events); at 65,536 LPs x 64 the array itself, read and
+// written once a window (41 of 96 us).  Its block steps -- sums by one warp, a batch
+// counted while it is written instead of searched for, keys placed by their rank in a run,
+// children kept in shared memory until their bucket's place is known, no 64-bit division --
+// took them from 30.9 and 113 us.
 // A batch's per-LP ranks (the order-sensitive hash needs each event's position in its
 // LP's sequence) come from a sort of (lp, position) keys: an event's rank is its LP's
 // count so far plus its distance from the first key of its LP.
@@ -730,7 +736,7 @@ __device__ bool hqg_insert_scan(const HqgDev& g, HqgState& q, const gpq_item* C,
 
 static constexpr uint32_t kHqgListCapI = kHqgTile;     // children per insert bucket
 static constexpr uint32_t kHqgListCapP = kHqgKeyTile;  // keys per LP-range bucket
-static constexpr uint32_t kHqgMaxBuckets = 160;        // >= the grid (one CTA per SM)
+static constexpr uint32_t kHqgMaxBuckets = 160;        // > the grid (one CTA per SM): the last word of pcnt counts a batch
 
 struct HqgLists {
   bool ins;     // this window's children are filed in the insert lists
@@ -874,9 +880,12 @@ __device__ bool hqg_bin_sort_items(const gpq_item* in, gpq_item* out, uint32_t n
   __syncthreads();
   const uint32_t t0 = s_tmin;
   const uint64_t span = ((uint64_t)(s_tmax - t0) + 1u) << 16;  // <= 2^48
-  auto bin_of = [t0, span, NB, L](const gpq_item& x) {
-    const uint64_t v = ((uint64_t)(gpq_f2u(x.ts) - t0) << 16) + (((uint64_t)x.lp << 16) / L);
-    return (uint32_t)(v * NB / span);  // v * NB < 2^61
+  // bin = v * NB / span and lp * 2^16 / L by reciprocals rounded down: still monotone and
+  // in range, and no 64-bit division per item (two were 6 of a 4 M-item window's 13 us here)
+  const uint64_t rec = (~0ull / span) * NB, lrec = (1ull << 48) / L;
+  auto bin_of = [t0, rec, lrec](const gpq_item& x) {
+    const uint64_t v = ((uint64_t)(gpq_f2u(x.ts) - t0) << 16) + ((x.lp * lrec) >> 32);
+    return (uint32_t)__umul64hi(v, rec);
   };
   for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) atomicAdd(&bins[bin_of(in[hqg_pad<HqgItemOps>(j)])], 1u);
   __syncthreads();
@@ -905,12 +914,13 @@ __device__ bool hqg_bin_sort_items(const gpq_item* in, gpq_item* out, uint32_t n
   return true;
 }
 
-// Groups the n (lp, position) keys of in (padded tile) by LP into out (padded tile): a
-// counting sort over the LP range [lp0, lp0 + W), then each LP's run sorted by position
-// (insertion sort, one thread per LP).  On return bins[b] is the end of LP lp0 + b's run
-// (its start: bins[b - 1], or 0).  Returns false, with out unusable, when W exceeds
-// kHqgBins or some LP has more than kHqgRunMax keys.  All threads.
-__device__ bool hqg_group_by_lp(const unsigned long long* in, unsigned long long* out, uint32_t n, uint32_t lp0,
+// Sorts the n (lp, position) keys of in (padded tile; tmp: another): a counting sort over
+// the LP range [lp0, lp0 + W), then each key placed in its LP's run by the number of
+// smaller positions there (every thread its own keys; an insertion sort by one thread per
+// LP took 19 us on runs of 25).  On return bins[b] is the end of LP lp0 + b's run (its
+// start: bins[b - 1], or 0).  Returns false, with in as it was, when W exceeds kHqgBins or
+// some LP has more than kHqgRunMax keys.  All threads.
+__device__ bool hqg_group_by_lp(unsigned long long* in, unsigned long long* tmp, uint32_t n, uint32_t lp0,
                                 uint32_t W, uint32_t* bins) {
   __shared__ int s_outside;
   if (W > kHqgBins || W == 0) return false;
@@ -930,20 +940,15 @@ __device__ bool hqg_group_by_lp(const unsigned long long* in, unsigned long long
   for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
     const unsigned long long k = in[hqg_pad<HqgKeyOps>(j)];
     const uint32_t pos = atomicAdd(&bins[(uint32_t)(k >> 32) - lp0], 1u);
-    if (pos < n) out[hqg_pad<HqgKeyOps>(pos)] = k;
+    if (pos < n) tmp[hqg_pad<HqgKeyOps>(pos)] = k;
   }
   __syncthreads();
-  for (uint32_t b = threadIdx.x; b < W; b += blockDim.x) {
-    const uint32_t e = bins[b], st = b ? bins[b - 1] : 0u;
-    for (uint32_t x = st + 1; x < e; ++x) {  // insertion sort of the run by position
-      const unsigned long long v = out[hqg_pad<HqgKeyOps>(x)];
-      uint32_t y = x;
-      while (y > st && out[hqg_pad<HqgKeyOps>(y - 1)] > v) {
-        out[hqg_pad<HqgKeyOps>(y)] = out[hqg_pad<HqgKeyOps>(y - 1)];
-        --y;
-      }
-      out[hqg_pad<HqgKeyOps>(y)] = v;
-    }
+  for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
+    const unsigned long long k = tmp[hqg_pad<HqgKeyOps>(j)];
+    const uint32_t b = (uint32_t)(k >> 32) - lp0, e = bins[b], st = b ? bins[b - 1] : 0u;
+    uint32_t r = st;
+    for (uint32_t x = st; x < e; ++x) r += tmp[hqg_pad<HqgKeyOps>(x)] < k ? 1u : 0u;
+    in[hqg_pad<HqgKeyOps>(r)] = k;
   }
   __syncthreads();
   return true;
@@ -954,11 +959,14 @@ __device__ bool hqg_group_by_lp(const unsigned long long* in, unsigned long long
 // each event folded into its LP's outputs in order (the per-LP sums of a warp's run added
 // by one lane), its child written to ch[base + position] and filed by `ins` (counted per
 // bucket in shared memory, one reservation per bucket, then written), the LP's count
-// advanced.  aux: kHqgBins words for the children's bucket slots.  All threads.
+// advanced.  slots: kHqgBins words for the children's bucket slots; stash: a free tile that
+// keeps the first kHqgStash children until their places are known.  All threads.
+static constexpr uint32_t kHqgStash = kHqgThreads * (kHqgKpt + 1) * sizeof(unsigned long long) / sizeof(gpq_item);
+
 template <class Seg>
 __device__ void hqg_process_keys(const PholdDev& d, const HqgDev& g, const gpq_item* root,
                                  const unsigned long long* K, uint32_t n, uint32_t base, const HqgIns& ins,
-                                 uint32_t* slots, Seg seg) {
+                                 uint32_t* slots, gpq_item* stash, Seg seg) {
   __shared__ uint32_t s_bc[kHqgMaxBuckets], s_gb[kHqgMaxBuckets];
   if (ins.on) {
     for (uint32_t k = threadIdx.x; k < ins.BI; k += blockDim.x) s_bc[k] = 0u;
@@ -985,6 +993,7 @@ __device__ void hqg_process_keys(const PholdDev& d, const HqgDev& g, const gpq_i
       if (ins.on && !direct && j < kHqgBins) {
         const uint32_t bk = hqg_bucket_of(ins.spl, ins.BI - 1, ch);
         slots[j] = (bk << 16) | atomicAdd(&s_bc[bk], 1u);
+        if (j < kHqgStash) stash[j] = ch;
       }
       if (ins.on && direct) chd = ch;
     }
@@ -1019,8 +1028,7 @@ __device__ void hqg_process_keys(const PholdDev& d, const HqgDev& g, const gpq_i
       s_gb[k] = s_bc[k] ? atomicAdd(&ins.icnt[k], s_bc[k]) : 0u;
     __syncthreads();
     for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
-      const uint32_t i = (uint32_t)K[hqg_pad<HqgKeyOps>(j)];
-      const gpq_item ch = g.h.ch[base + i];
+      const gpq_item ch = j < kHqgStash ? stash[j] : g.h.ch[base + (uint32_t)K[hqg_pad<HqgKeyOps>(j)]];
       if (j < kHqgBins) {
         const uint32_t sv = slots[j], bk = sv >> 16, slot = s_gb[bk] + (sv & 0xffffu);
         if (slot < kHqgListCapI) ins.ilist[(size_t)bk * kHqgListCapI + slot] = ch;
@@ -1035,26 +1043,32 @@ __device__ void hqg_process_keys(const PholdDev& d, const HqgDev& g, const gpq_i
 }
 
 // Sorts the n keys of sa (an LP range of W LPs from lp0) for hqg_process_keys and runs it:
-// grouped by LP when it can, else the block merge sort.
+// by LP when it can, else -- and up to kHqgRankKeysMax keys, which are placed by rank in one
+// step -- by the block sort.  The line: the rank sort reads every key once per key, so it
+// grows with n^2 (5,575 LPs x 35, about 300 keys a CTA: 3.45 ms grouped, 4.96 ms by rank),
+// while the counting sort's five block steps cost about 2 us whatever n is.
+static constexpr uint32_t kHqgRankKeysMax = 128;
+
 __device__ void hqg_sort_and_process(const PholdDev& d, const HqgDev& g, const gpq_item* root,
                                      unsigned long long* sa, unsigned long long* sb, uint32_t n, uint32_t lp0,
                                      uint32_t W, uint32_t base, const HqgIns& ins, uint32_t* aux) {
   uint32_t* bins = aux;
   uint32_t* slots = aux + kHqgBins;
-  if (hqg_group_by_lp(sa, sb, n, lp0, W, bins)) {
-    hqg_process_keys(d, g, root, sb, n, base, ins, slots,
+  if (n > kHqgRankKeysMax && hqg_group_by_lp(sa, sb, n, lp0, W, bins)) {
+    hqg_process_keys(d, g, root, sa, n, base, ins, slots, reinterpret_cast<gpq_item*>(sb),
                      [bins, lp0](uint32_t, uint32_t lp) { return lp > lp0 ? bins[lp - lp0 - 1] : 0u; });
   } else {
     const unsigned long long* K = hqg_cta_sort<HqgKeyOps>(sa, sb, n);
-    hqg_process_keys(d, g, root, K, n, base, ins, slots, [K](uint32_t j, uint32_t lp) {
-      const unsigned long long lo_key = (unsigned long long)lp << 32;
-      uint32_t l = 0, h = j;
-      while (l < h) {
-        const uint32_t mid = (l + h) >> 1;
-        if (K[hqg_pad<HqgKeyOps>(mid)] < lo_key) l = mid + 1; else h = mid;
-      }
-      return l;
-    });
+    hqg_process_keys(d, g, root, K, n, base, ins, slots, reinterpret_cast<gpq_item*>(K == sa ? sb : sa),
+                     [K](uint32_t j, uint32_t lp) {
+                       const unsigned long long lo_key = (unsigned long long)lp << 32;
+                       uint32_t l = 0, h = j;
+                       while (l < h) {
+                         const uint32_t mid = (l + h) >> 1;
+                         if (K[hqg_pad<HqgKeyOps>(mid)] < lo_key) l = mid + 1; else h = mid;
+                       }
+                       return l;
+                     });
   }
 }
 
@@ -1167,16 +1181,19 @@ __device__ void hqg_file_range(const HqgDev& g, const gpq_item* root, uint32_t l
 // items right after the first -- into the root's other buffer.  Returns false, with
 // nothing written, when a list overflowed.
 //
+// The new root's head is the smaller of R's head and the smallest child (in the first
+// non-empty list), which fixes the next window's bound; each CTA adds its outputs below it
+// to *pre.below, so that the next window knows its batch without a search.
+//
 // pre.on: the next window's batch is also filed into its LP-range lists (pre.BP ranges,
-// counts pre.pc) here, so that the window needs no filing phase: the new root's head is the
-// smaller of R's head and the smallest child (in the first non-empty list), which fixes the
-// window's bound; each CTA's outputs below it are a prefix of its output range, filed by
-// that CTA after its merge.
+// counts pre.pc) here, so that the window needs no filing phase: each CTA's outputs below
+// the bound are a prefix of its output range, filed by that CTA after its merge.
 struct HqgPre {
   bool on;
   float la, T;   // lookahead and end time: the bound is min(head + la, T)
   uint32_t BP;   // LP ranges
   uint32_t* pc;  // their counts (zeroed before the window)
+  uint32_t* below;  // items below the next window's bound (zeroed before the window)
 };
 
 __device__ bool hqg_insert_lists(const HqgDev& g, HqgState& q, uint32_t nch, uint32_t BI, const uint32_t* ic,
@@ -1187,39 +1204,47 @@ __device__ bool hqg_insert_lists(const HqgDev& g, HqgState& q, uint32_t nch, uin
   uint32_t* aux = hqg_aux(smem);
   const gpq_item* R = q.root + q.off;
   const uint32_t nr = q.cnt0;
-  for (uint32_t k = threadIdx.x; k < BI; k += blockDim.x) s_pre[k] = ic[k];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t run = 0;
-    int ovf = 0;
-    for (uint32_t k = 0; k < BI; ++k) {
+  if (threadIdx.x < 32u) {  // the lists' exclusive sums, a run of them per lane
+    const uint32_t per = (BI + 31u) / 32u, k0 = min(BI, threadIdx.x * per), k1 = min(BI, k0 + per);
+    uint32_t sum = 0, first = BI;
+    bool ovf = false;
+    for (uint32_t k = k0; k < k1; ++k) {
+      const uint32_t v = ic[k];
+      ovf |= v > kHqgListCapI;
+      if (v != 0u) first = min(first, k);
+      s_pre[k] = v;
+      sum += v;
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(GPQ_FULL_MASK, incl, o);
+      if (threadIdx.x >= (uint32_t)o) incl += u;
+    }
+    uint32_t run = incl - sum;
+    for (uint32_t k = k0; k < k1; ++k) {
       const uint32_t v = s_pre[k];
-      ovf |= v > kHqgListCapI ? 1 : 0;
       s_pre[k] = run;
       run += v;
     }
-    s_pre[BI] = run;
-    s_ovf = ovf || run != nch;
+    first = warp_min_u32(first);
+    const bool any = __any_sync(GPQ_FULL_MASK, ovf);
+    if (threadIdx.x == 31u) {
+      s_pre[BI] = incl;
+      s_ovf = any || incl != nch;
+      s_b0 = first;  // the first non-empty list
+    }
   }
   __syncthreads();
   if (s_ovf) return false;  // the same decision in every block: nothing written
-  uint32_t lim = 0;  // pre.on: the next window's bound (ts bits), the same in every block
-  if (pre.on) {
-    if (threadIdx.x == 0) {
-      uint32_t b0 = BI;
-      for (uint32_t k = 0; k < BI && b0 == BI; ++k)
-        if (s_pre[k + 1] > s_pre[k]) b0 = k;
-      s_b0 = b0;
-    }
-    __syncthreads();
-    uint32_t mn = (threadIdx.x == 0 && nr > 0) ? gpq_f2u(R[0].ts) : kInfBits;
-    if (s_b0 < BI) {
-      const gpq_item* l0 = g.ilist + (size_t)s_b0 * kHqgListCapI;
-      for (uint32_t j = threadIdx.x; j < s_pre[s_b0 + 1] - s_pre[s_b0]; j += blockDim.x) mn = min(mn, gpq_f2u(l0[j].ts));
-    }
-    mn = block_min_u32(mn, s_red);
-    lim = min(gpq_f2u(GPQ_FADD(gpq_u2f(mn), pre.la)), gpq_f2u(pre.T));
+  // the next window's bound (ts bits), the same in every block
+  uint32_t mn = (threadIdx.x == 0 && nr > 0) ? gpq_f2u(R[0].ts) : kInfBits;
+  if (s_b0 < BI) {
+    const gpq_item* l0 = g.ilist + (size_t)s_b0 * kHqgListCapI;
+    for (uint32_t j = threadIdx.x; j < s_pre[s_b0 + 1] - s_pre[s_b0]; j += blockDim.x) mn = min(mn, gpq_f2u(l0[j].ts));
   }
+  mn = block_min_u32(mn, s_red);
+  const uint32_t lim = min(gpq_f2u(GPQ_FADD(gpq_u2f(mn), pre.la)), gpq_f2u(pre.T));
   gpq_item* sa = reinterpret_cast<gpq_item*>(smem);
   gpq_item* sb = sa + hqg_tile_cap<HqgItemOps>();
   gpq_item* out = q.spare;
@@ -1290,12 +1315,20 @@ __device__ bool hqg_insert_lists(const HqgDev& g, HqgState& q, uint32_t nch, uin
     }
     for (uint32_t j = cpos + threadIdx.x; j < nc; j += blockDim.x) out[base + nrb + j] = X[hqg_pad<HqgItemOps>(j)];
     __syncthreads();
-    if (pre.on) {  // this CTA's outputs below the bound: R's and the children's below it
-      const uint32_t nR = hqg_cta_search(0, nrb, [R, r0, lim](uint32_t i) { return gpq_f2u(R[r0 + i].ts) >= lim; });
-      const uint32_t nX =
-          hqg_cta_search(0, nc, [X, lim](uint32_t i) { return gpq_f2u(X[hqg_pad<HqgItemOps>(i)].ts) >= lim; });
-      hqg_file_range(g, out, base, base + nR + nX, pre.BP, pre.pc, L, aux);
+    // this CTA's outputs below the bound: R's and the children's below it
+    uint32_t nR = 0, nX = 0;
+    if (nrb > 0 && gpq_f2u(R[r0].ts) < lim) {
+      nR = nrb;
+      if (gpq_f2u(R[r1 - 1u].ts) >= lim)
+        nR = hqg_cta_search(0, nrb, [R, r0, lim](uint32_t i) { return gpq_f2u(R[r0 + i].ts) >= lim; });
     }
+    for (uint32_t hi = nc; nX < hi;) {
+      const uint32_t mid = (nX + hi) >> 1;
+      if (gpq_f2u(X[hqg_pad<HqgItemOps>(mid)].ts) < lim) nX = mid + 1; else hi = mid;
+    }
+    if (threadIdx.x == 0 && nR + nX) atomicAdd(pre.below, nR + nX);
+    if (pre.on) hqg_file_range(g, out, base, base + nR + nX, pre.BP, pre.pc, L, aux);
+    __syncthreads();
   }
   if (!hqg_bar(s)) return false;
   q.swap_root();
@@ -1334,6 +1367,7 @@ static __global__ void __launch_bounds__(kHqgThreads, 1) hqg_phold_kernel(PholdD
   uint32_t steps = 0, nch = 0, ovf_seen = 0;
   uint32_t c_last = 0;    // size of the last batch
   bool prefiled = false;  // this window's batch was filed by the insert phase (pre_bp ranges)
+  bool counted = false;   // ... and counted
   uint32_t pre_bp = 0;
   HqgLists lists{false, 0u};
   __shared__ gpq_item s_spl[kHqgMaxBuckets];
@@ -1355,9 +1389,11 @@ static __global__ void __launch_bounds__(kHqgThreads, 1) hqg_phold_kernel(PholdD
         pre.T = d.p.end_time;
         pre.BP = min(gridDim.x, max(1u, c_last / 64u));
         pre.pc = g.pcnt + ((steps + 1u) & 1u) * kHqgMaxBuckets;
+        pre.below = pre.pc + kHqgMaxBuckets - 1u;
         done = hqg_insert_lists(g, q, nch, lists.BI, g.icnt + (steps & 1u) * kHqgMaxBuckets, d.L, pre, smem, s);
         if (!s.ok) break;
         prefiled = done && pre.on;
+        counted = done;
         pre_bp = pre.BP;
       }
       lists.ins = false;
@@ -1380,9 +1416,12 @@ static __global__ void __launch_bounds__(kHqgThreads, 1) hqg_phold_kernel(PholdD
     ++steps;
     while (s.ok) {  // batches of the window
       const gpq_item* root = q.root + q.off;
-      const uint32_t c = hqg_cta_search(0, q.cnt0, [root, lim](uint32_t i) { return gpq_f2u(root[i].ts) >= lim; });
+      const uint32_t c =
+          counted ? ld_relaxed_u32(g.pcnt + (steps & 1u) * kHqgMaxBuckets + kHqgMaxBuckets - 1u)
+                  : hqg_cta_search(0, q.cnt0, [root, lim](uint32_t i) { return gpq_f2u(root[i].ts) >= lim; });
       const bool use_pre = prefiled;  // only the window's first batch
       prefiled = false;
+      counted = false;
       if (c == 0) break;
       // LP-range lists for the batch (a heap whose root holds every item; other heaps scan
       // the batch in each CTA or take the general path)
@@ -1400,17 +1439,21 @@ static __global__ void __launch_bounds__(kHqgThreads, 1) hqg_phold_kernel(PholdD
           hqg_file_batch(d, g, root, c, BP, pc, smem, s);
           if (!s.ok) break;
         }
-        for (uint32_t k = threadIdx.x; k < BP; k += blockDim.x) s_pc[k] = ld_relaxed_u32(&pc[k]);
-        __syncthreads();
-        if (threadIdx.x == 0) {
+        if (threadIdx.x < 32u) {
           uint32_t sum = 0;
-          int ovf = 0;
-          for (uint32_t k = 0; k < BP; ++k) {
-            sum += s_pc[k];
-            ovf |= s_pc[k] > kHqgListCapP ? 1 : 0;
+          bool ovf = false;
+          for (uint32_t k = threadIdx.x; k < BP; k += 32u) {
+            const uint32_t v = ld_relaxed_u32(&pc[k]);
+            s_pc[k] = v;
+            sum += v;
+            ovf |= v > kHqgListCapP;
           }
-          s_pc_sum = sum;
-          s_pc_ovf = ovf;
+          sum = warp_sum_u32(sum);
+          ovf = __any_sync(GPQ_FULL_MASK, ovf);
+          if (threadIdx.x == 0) {
+            s_pc_sum = sum;
+            s_pc_ovf = ovf;
+          }
         }
         __syncthreads();
         from_lists = !s_pc_ovf && s_pc_sum == c;
@@ -1461,6 +1504,7 @@ static __global__ void __launch_bounds__(kHqgThreads, 1) hqg_phold_kernel(PholdD
       nch += c;
       q.off += c;
       q.cnt0 -= c;
+      if (q.last == 0) break;  // the root held every item: the batch was the whole window
       if (!hqg_refill(g, q, smem, s)) break;
     }
   }

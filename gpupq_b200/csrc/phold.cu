@@ -258,7 +258,7 @@ gpq_status gpq_phold_create(const gpq_phold_config* cfg_in, gpq_phold** out) {
         gpq::set_last_error("heap queue: the grid kernel does not fit on an SM");
         return fail(GPQ_ERR_INVALID);
       }
-      h->hqg_blocks = std::min<uint32_t>((uint32_t)h->num_sms, kHqgMaxBuckets);  // one CTA per SM
+      h->hqg_blocks = std::min<uint32_t>((uint32_t)h->num_sms, kHqgMaxBuckets - 1);  // one CTA per SM
     } else {
       TRY(gpq::raise_smem_limit(hq_phold_kernel, (int)hq_smem_bytes(r)));
     }

@@ -151,3 +151,27 @@ def test_bucket_overflow_falls_back(gpu_lib):
         assert r[k] == r0[k], k
     for k in ("count", "csum", "ohash"):
         assert np.array_equal(s[k], s0[k]), k
+
+
+@pytest.mark.parametrize("num_lps,per,la", [
+    (512, 16, 0.05),    # a few keys per CTA: placed by rank
+    (9665, 3, 2.0),     # about 128 keys per CTA: both sides of the rank sort's limit
+    (40, 2000, 0.25),   # runs of an LP around 64 keys: grouped by LP, and too long for it
+    (301, 400, 1.0),    # more children per CTA than the shared copy keeps
+])
+@pytest.mark.parametrize("queue", ["hq", "gaq"])
+def test_batch_sizes(gpu_lib, queue, num_lps, per, la):
+    """The root holds every item; batches per CTA around the edges of the sorts' forms, in one
+    launch and in single windows (whose batch the launch before has not counted)."""
+    cfgd = dict(num_lps=num_lps, events_per_lp=per, lookahead=la, end_time=10 * la, seed=23, dest_mode=1, ring_width=5)
+    o = _oracle(cfgd)
+    cfg = G.make_phold_config(**cfgd, queue=queue, capacity=1 << max(6, (per - 1).bit_length()))
+    for steps in (None, 1):
+        with G.Phold(cfg) as h:
+            h.populate()
+            if steps is None:
+                h.run()
+            else:
+                while not h.step(steps):
+                    pass
+            _assert_same(h.result(), h.lp_stats(), o)
