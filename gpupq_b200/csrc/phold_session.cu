@@ -29,6 +29,7 @@ struct gpq_phold_session {
   uint32_t* wr = nullptr;
   gpq_item* ibuf = nullptr;
   uint32_t* icnt = nullptr;
+  uint32_t* lmin = nullptr;
   uint32_t* count = nullptr;
   unsigned long long* csum = nullptr;
   unsigned long long* ohash = nullptr;
@@ -60,16 +61,6 @@ cudaError_t dmalloc(T** p, uint64_t n) {
   return cudaMalloc(p, std::max<uint64_t>(n, 1) * sizeof(T));
 }
 
-const void* pm_kernel(uint32_t group) {
-  switch (group) {
-    case 4: return (const void*)pm_persistent_kernel<4>;
-    case 8: return (const void*)pm_persistent_kernel<8>;
-    case 16: return (const void*)pm_persistent_kernel<16>;
-    case 32: return (const void*)pm_persistent_kernel<32>;
-  }
-  return nullptr;
-}
-
 PmDev session_dev(const gpq_phold_session* s) {
   PmDev d{};
   d.inst = s->inst;
@@ -86,6 +77,7 @@ PmDev session_dev(const gpq_phold_session* s) {
   d.ibuf = s->ibuf;
   d.icnt = s->icnt;
   d.ibc = s->ibc;
+  d.lmin = s->lmin;
   d.max_lps = s->max_lps;
   d.count = s->count;
   d.csum = s->csum;
@@ -371,6 +363,7 @@ gpq_status gpq_phold_session_restore(gpq_phold_session* s, const void* buf, uint
     if (r.second) GPQ_CUDA_TRY(cudaMemcpyAsync(r.first, p, r.second, cudaMemcpyHostToDevice, st));
     p += r.second;
   }
+  if (s->lmin) GPQ_CUDA_TRY(cudaMemsetAsync(s->lmin, 0, (size_t)k[1] * sizeof(uint32_t), st));  // not known
   // slots and LPs above the snapshot's highest ones are free
   if (k[0] < s->max_inst) GPQ_CUDA_TRY(cudaMemsetAsync(s->on + k[0], 0, s->max_inst - k[0], st));
   if (k[1] < s->max_lps)
@@ -399,7 +392,8 @@ gpq_status gpq_phold_session_create(uint32_t max_lps, uint32_t capacity, uint32_
   GPQ_CHECK_ARG(max_lps >= 1 && max_instances >= 1 && max_instances <= (1u << 20), "need max_lps >= 1, 1 <= max_instances <= 2^20");
   GPQ_CHECK_ARG(gpq::is_pow2(capacity) && capacity >= 8 && capacity <= (1u << 20), "capacity must be a power of two in [8, 2^20]");
   GPQ_CHECK_ARG(insert_capacity >= 1 && insert_capacity <= 4096, "insert_capacity in [1, 4096]");
-  GPQ_CHECK_ARG(pm_kernel(lanes_per_lp) != nullptr, "lanes_per_lp must be 4, 8, 16 or 32");
+  GPQ_CHECK_ARG(lanes_per_lp == 4 || lanes_per_lp == 8 || lanes_per_lp == 16 || lanes_per_lp == 32,
+                "lanes_per_lp must be 4, 8, 16 or 32");
   gpq_phold_session* s = new (std::nothrow) gpq_phold_session();
   if (!s) return GPQ_ERR_NOMEM;
   s->max_lps = max_lps;
@@ -417,14 +411,25 @@ gpq_status gpq_phold_session_create(uint32_t max_lps, uint32_t capacity, uint32_
   if (e == cudaSuccess) e = dmalloc(&s->wr, max_lps);
   if (e == cudaSuccess) e = dmalloc(&s->ibuf, 2ull * max_lps * insert_capacity);
   if (e == cudaSuccess) e = dmalloc(&s->icnt, 2ull * max_lps);
+  if (e == cudaSuccess) e = dmalloc(&s->lmin, max_lps);
   if (e == cudaSuccess) e = cudaMemsetAsync(s->icnt, 0, 2ull * max_lps * 4, s->own);
   if (e != cudaSuccess) {
     set_last_error("gpq_phold_session_create: %s", cudaGetErrorString(e));
     gpq_phold_session_destroy(s);
     return e == cudaErrorMemoryAllocation ? GPQ_ERR_NOMEM : GPQ_ERR_CUDA;
   }
-  s->kern = pm_kernel(s->group);
-  s->smem = (size_t)(s->block / s->group) * laq_group_smem_bytes(s->ibc, s->group);
+  {  // the insert buffers of 256 / lanes_per_lp LPs, staged at once, bound the insert capacity
+    int dev = 0, limit = 0;
+    cudaError_t q = cudaGetDevice(&dev);
+    if (q == cudaSuccess) q = cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (q != cudaSuccess || (size_t)(s->block / s->group) * laq_group_smem_bytes(s->ibc, s->group) > (size_t)limit) {
+      set_last_error("gpq_phold_session_create: insert_capacity %u too large for %u lanes per LP", s->ibc, s->group);
+      gpq_phold_session_destroy(s);
+      return GPQ_ERR_CUDA;
+    }
+  }
+  s->kern = (const void*)pm_persistent_kernel;
+  s->smem = (s->block / 32) * pm_sel_warp_bytes();
   const gpq_status fs = finish_create(s, max_instances);
   if (fs != GPQ_OK) {
     gpq_phold_session_destroy(s);
@@ -484,7 +489,7 @@ gpq_status gpq_phold_session_create_bucketed(uint32_t max_lps, uint32_t buckets,
 gpq_status gpq_phold_session_destroy(gpq_phold_session* s) {
   if (!s) return GPQ_OK;
   void* bufs[] = {s->inst,   s->mins,   s->errs,     s->on,       s->lp_inst,   s->ring,     s->rd,    s->wr,
-                  s->ibuf,   s->icnt,   s->count,    s->csum,     s->ohash,     s->ctl,      s->list,  s->list_n,
+                  s->ibuf,   s->icnt,   s->lmin,   s->count,    s->csum,     s->ohash,     s->ctl,      s->list,  s->list_n,
                   s->acc,    s->staged, s->b.q.keys, s->b.q.cnt, s->b.q.spill, s->b.q.scnt, s->b.wj, s->b.fin};
   for (void* p : bufs)
     if (p) cudaFree(p);

@@ -158,3 +158,36 @@ def test_session_snapshot_rejects_other_parameters(gpu_lib):
     with G.PholdSession(max_lps=1000, max_instances=4) as t:
         with pytest.raises(G.GpqError):
             t.restore(snap[:-5])
+
+
+@pytest.mark.parametrize("shape", [
+    # (LPs, events per LP, lookahead, end time) of the runs; capacity; insert capacity; lanes
+    ([(700, 44, 30.0, 90.0), (61, 46, 30.0, 90.0), (33, 1, 0.3, 9.0)], 256, 128, 8),  # about a list of safe events
+    ([(40, 200, 6.0, 30.0), (9, 130, 0.01, 0.5)], 512, 400, 16),                      # more than a list
+    ([(3, 740, 9.0, 30.0), (2, 1000, 9.0, 30.0), (5, 16, 0.5, 20.0)], 2048, 1150, 32),  # about and above the wide list
+    ([(20001, 24, 0.4, 4.0), (3, 8, 2.0, 8.0), (500, 20, 0.001, 0.05)], 64, 64, 8),   # eight LPs a turn; idle LPs
+    ([(5, 4, 1.0, 10.0 + 0.1 * i) for i in range(300)], 64, 64, 4),                   # more runs than the bounds' table
+])
+def test_selection_sizes(gpu_lib, shape):
+    """Windows whose safe events fit an LP's list, outgrow it and outgrow the warp's space."""
+    runs, capacity, insert, lanes = shape
+    cfgs = [G.make_phold_config(L, per, la, T, 70 + i) for i, (L, per, la, T) in enumerate(runs)]
+    with G.PholdSession(max_lps=sum(c.num_lps for c in cfgs), max_instances=len(cfgs), capacity=capacity,
+                        insert_capacity=insert, lanes_per_lp=lanes) as s:
+        slot_of = {s.admit(c): i for i, c in enumerate(cfgs)}
+        s.step(3)  # then the rest: rings left by one launch, taken up by the next
+        s.step(0)
+        got = {slot_of[sl]: r for sl, r in s.collect()}
+    for i, c in enumerate(cfgs):
+        alone = G.make_phold_config(c.num_lps, c.events_per_lp, c.lookahead, c.end_time, c.seed, queue="hq",
+                                    capacity=capacity)
+        with G.Phold(alone) as h:
+            h.populate()
+            h.run()
+            _same(got[i], h.result())
+
+
+def test_insert_capacity_too_large_is_refused(gpu_lib):
+    with pytest.raises(G.GpqError):
+        G.PholdSession(max_lps=8, max_instances=1, insert_capacity=2048, lanes_per_lp=8)
+    G.PholdSession(max_lps=8, max_instances=1, insert_capacity=1024, lanes_per_lp=32).close()
