@@ -94,18 +94,22 @@ inline uint32_t lsq_lanes(uint32_t num_lps) {
   return 1;
 }
 
-// Default lanes per LP of the sorted local array queue (laq_mode 0 and 1).  With few LPs a
-// window is one LP's chain of dependent steps, which more lanes shorten, as long as one
-// wave of CTAs holds them all; between one and about three waves of 8-lane groups the last
-// wave is short and 16 lanes even it out; beyond that the CTAs' throughput counts and 8
-// lanes cost least.  Measured (us a window with 8 / 16 / 32 lanes): 1,024 LPs x 16 events
-// 12.2 / 9.0 / 7.5, 2,048 x 16 12.7 / 9.4 / 8.3, 4,096 x 16 13.1 / 10.2 / 11.7, 8,192 x 16
-// 14.7 / 15.5 / 15.4, 20,011 x 32 29.2 / 27.6 / 31.5, 44,133 x 60 66.7 / 65.5 / 71.6,
-// 65,536 x 30 65.9 / 73.6 / 90.2.
-inline uint32_t laq_lanes(uint32_t num_lps) {
-  if (num_lps <= 2048) return 32;
-  if (num_lps <= 4096) return 16;
-  return num_lps > 14208 && num_lps <= 48000 ? 16 : 8;
+// Default lanes per LP of the sorted local array queue (laq_mode 0 and 1).  A wave of CTAs
+// holds 14,208 LPs with 8 lanes each, 7,104 with 16, 3,552 with 32.  In one wave a window is
+// one LP's chain of dependent steps, which more lanes shorten when the LP has several
+// events; between one and one and a half waves of 8 lanes, three short rounds of 16 beat two
+// long ones; otherwise the fixed steps per LP count and 8 lanes cost least.  Measured (us a
+// window, 8 / 16 / 32 lanes; events per LP and window): 1,024 LPs 6.7 / 6.3 / 5.7 (0.4),
+// 12.1 / 9.0 / 7.6 (8); 3,000 7.3 / 7.2 / 7.2 (0.8), 12.8 / 9.7 / 9.1 (8); 7,000 8.2 / 8.8
+// (0.8), 10.7 / 9.6 (3), 17.1 / 12.5 (11); 7,500 17.3 / 18.6 (11); 21,000 16.6 / 17.0 (3),
+// 26.0 / 22.4 (6), 55.0 / 46.4 (21); 24,000 29.5 / 34.0 (11); 40,000 17.2 / 25.9 (0.8),
+// 44.1 / 50.4 (11); 65,536 70.4 / 79.1 (11).
+inline uint32_t laq_lanes(const gpq_phold_config& c) {
+  const uint32_t L = c.num_lps;
+  const double events = (double)c.events_per_lp * c.lookahead / (1.0 + c.lookahead);
+  if (L <= 2048 || (L <= 3552 && events >= 5.0)) return 32;
+  if (L <= 4096 || (L <= 7104 && events >= 2.5)) return 16;
+  return L > 14208 && L <= 21312 && events >= 5.0 ? 16 : 8;
 }
 
 // Whether the local heap queue takes a warp per LP and a window's items in one piece
@@ -119,12 +123,12 @@ inline bool lhq_warp(const gpq_phold_config& c) {
   return c.num_lps <= 4096 || (double)c.events_per_lp * c.lookahead / (1.0 + c.lookahead) >= 7.5;
 }
 
-// Lanes per LP that a run uses: the asked-for number, or by the number of LPs.  `c` is the
+// Lanes per LP that a run uses: the asked-for number, or by the rules above.  `c` is the
 // normalized configuration, which goes into snapshots and keeps 8 (splay queue: 1) for the
 // default, so that a run's state goes between handles whatever their lanes.
 inline uint32_t run_lanes(const gpq_phold_config& c, uint32_t asked) {
   if (c.queue_kind == GPQ_QUEUE_LSQ) return lsq_lanes(c.num_lps);
-  if (c.queue_kind == GPQ_QUEUE_LAQ && c.laq_mode != 2 && asked == 0) return laq_lanes(c.num_lps);
+  if (c.queue_kind == GPQ_QUEUE_LAQ && c.laq_mode != 2 && asked == 0) return laq_lanes(c);
   return c.lanes_per_lp;
 }
 

@@ -44,6 +44,13 @@ def test_sorted_array_lanes(gpu_lib, lps):
         _check(dict(num_lps=lps, events_per_lp=9, lookahead=0.4, end_time=4.0, seed=lps, dest_mode=0), "laq", loop=loop)
 
 
+@pytest.mark.parametrize("lps", [2049, 3552, 3553, 7104, 7105, 14209, 21312, 21313])
+@pytest.mark.parametrize("per", [5, 24])
+def test_sorted_array_lanes_by_events(gpu_lib, lps, per):
+    """1.4 and 6.9 events per LP and window, around the waves of 32, 16 and 8 lanes."""
+    _check(dict(num_lps=lps, events_per_lp=per, lookahead=0.4, end_time=3.0, seed=lps, dest_mode=0), "laq")
+
+
 @pytest.mark.parametrize("lps,per,la,end,ring", [
     (1, 1, 0.5, 30.0, 0), (40, 1, 0.01, 3.0, 1), (4096, 9, 0.4, 6.0, 0), (4097, 9, 0.4, 6.0, 0), (4500, 17, 0.8, 8.0, 0),
     (300, 9, 3.0, 30.0, 1),     # most of a heap safe in every window
