@@ -209,8 +209,8 @@ __device__ __forceinline__ uint32_t lab_process_event(const LabCtx& x, const Lab
   const uint32_t idx = e.aux & 0xffffu;
   const uint32_t tb = gpq_f2u(e.ts);
   const uint64_t h = gpq_ev_hash(e.id, tb);
-  atomicAdd(&st.csum[slot], (unsigned long long)h);
-  atomicAdd(&st.ohash[slot], (unsigned long long)gpq_seq_hash(h, (uint64_t)st.seq0[slot] + idx));
+  shared_add_u64(&st.csum[slot], h);
+  shared_add_u64(&st.ohash[slot], gpq_seq_hash(h, (uint64_t)st.seq0[slot] + idx));
   const gpq_item ch = lab_child(x, e);
   const uint32_t cb = gpq_f2u(ch.ts);
   if (!(kShard && lab_handover(x, q, w, ch))) lab_push(x, q, ch.lp, lab_key(cb, ch.id), lab_bucket(cb, w.inv_w), w);
@@ -1005,8 +1005,8 @@ static __device__ uint32_t lab_warp_window(const LabCtx& x, const LabDev& q, con
     const uint32_t ns = min(sm.misc[0], kLabItemStageCap);
     auto get = [&](uint32_t y) { return sm.stage[y]; };
     auto put = [&](uint32_t, uint32_t slot, uint64_t h, uint64_t o) {
-      atomicAdd(&st.csum[slot], (unsigned long long)h);
-      atomicAdd(&st.ohash[slot], (unsigned long long)o);
+      shared_add_u64(&st.csum[slot], h);
+      shared_add_u64(&st.ohash[slot], o);
     };
     for (uint32_t x0 = lane; x0 < ns; x0 += 128u) mn = min(mn, lab_event_batch<kShard>(x, q, st, ns, x0, 32u, w, get, put));
   }
