@@ -626,12 +626,12 @@ __device__ __forceinline__ uint32_t lab_scan_above(const LabDev& q, uint32_t lp,
 }
 
 // Events x0, x0 + stride, ... (up to four per thread) of a staging area (`get(x)` returns
-// staged event x, or one whose aux is kStageHole): hashes (`put(x, slot, h, oh)` takes event
-// x's) and the children first, then all bucket reservations (independent atomics in flight
-// together), then the stores.  Returns the children's minimum.
-template <bool kShard, class Get, class Put>
-__device__ __forceinline__ uint32_t lab_event_batch(const LabCtx& x, const LabDev& q, const PholdStage& st, uint32_t ns,
-                                                    uint32_t x0, uint32_t stride, const LabWin& w, Get get, Put put) {
+// staged event x, or one whose aux is kStageHole): hashes into the LP accumulators and the
+// children first, then all bucket reservations (independent atomics in flight together),
+// then the stores.  Returns the children's minimum.
+template <bool kShard, class Get>
+__device__ __forceinline__ uint32_t lab_event_batch(const LabCtx& x, const LabDev& q, const PholdStage& st,
+                                                    uint32_t ns, uint32_t x0, uint32_t stride, const LabWin& w, Get get) {
   constexpr int U = 4;
   const uint32_t nbm = (1u << q.nb_log2) - 1u, C = 1u << q.c_log2;
   unsigned long long key[U];
@@ -646,7 +646,8 @@ __device__ __forceinline__ uint32_t lab_event_batch(const LabCtx& x, const LabDe
       if (e.aux != kStageHole) {
         const uint32_t slot = e.aux >> 16, idx = e.aux & 0xffffu, tb = gpq_f2u(e.ts);
         const uint64_t h = gpq_ev_hash(e.id, tb);
-        put(xi, slot, h, gpq_seq_hash(h, (uint64_t)st.seq0[slot] + idx));
+        shared_add_u64(&st.csum[slot], h);
+        shared_add_u64(&st.ohash[slot], gpq_seq_hash(h, (uint64_t)st.seq0[slot] + idx));
         const gpq_item ch = lab_child(x, e);
         const uint32_t cb = gpq_f2u(ch.ts);
         mn = min(mn, cb);
@@ -984,31 +985,11 @@ static __device__ uint32_t lab_warp_window(const LabCtx& x, const LabDev& q, con
       e.aux = (lpi << 16) | ((c >> 8) & 0xffu);
       return e;
     };
-    // an event leaves its hashes in its candidate's place and in the safe lists' space, and
-    // two lanes an LP add them up afterwards: a 64-bit shared atomic per hash is a loop of
-    // compare-and-swaps, one turn for every event of the LP in the warp (65,536 LPs x 64,
-    // lookahead 0.1: 30.4 us a window with the atomics, 27.7 without)
-    unsigned long long* const oh = reinterpret_cast<unsigned long long*>(sm.sidx);
-    auto put = [&](uint32_t y, uint32_t, uint64_t h, uint64_t o) {
-      sm.cand[sm.cstage[y] & 0xffu] = h;
-      oh[y] = o;
-    };
-    for (uint32_t x0 = lane; x0 < ns; x0 += 128u) mn = min(mn, lab_event_batch<kShard>(x, q, st, ns, x0, 32u, w, get, put));
-    __syncwarp();
-    if (lane < 2u * n) {
-      const uint32_t lpi = lane >> 1, e = min(sm.lp_soff[lpi + 1u], kLabStageCap);
-      unsigned long long sum = 0;
-      for (uint32_t y = sm.lp_soff[lpi]; y < e; ++y) sum += (lane & 1u) ? oh[y] : sm.cand[sm.cstage[y] & 0xffu];
-      ((lane & 1u) ? sm.ls_ohash : sm.ls_csum)[lpi] += sum;
-    }
+    for (uint32_t x0 = lane; x0 < ns; x0 += 128u) mn = min(mn, lab_event_batch<kShard>(x, q, st, ns, x0, 32u, w, get));
   } else {
     const uint32_t ns = min(sm.misc[0], kLabItemStageCap);
     auto get = [&](uint32_t y) { return sm.stage[y]; };
-    auto put = [&](uint32_t, uint32_t slot, uint64_t h, uint64_t o) {
-      shared_add_u64(&st.csum[slot], h);
-      shared_add_u64(&st.ohash[slot], o);
-    };
-    for (uint32_t x0 = lane; x0 < ns; x0 += 128u) mn = min(mn, lab_event_batch<kShard>(x, q, st, ns, x0, 32u, w, get, put));
+    for (uint32_t x0 = lane; x0 < ns; x0 += 128u) mn = min(mn, lab_event_batch<kShard>(x, q, st, ns, x0, 32u, w, get));
   }
   if (common) {
     if (scan_lpi != ~0u && scan_min != kInfBits) atomicMin(&sm.lp_nmin[scan_lpi], scan_min);

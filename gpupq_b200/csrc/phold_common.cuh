@@ -101,7 +101,8 @@ struct PholdStage {
 // high one's): a 64-bit shared atomic is a loop of compare-and-swaps, one turn for every lane
 // of the warp that adds to the same LP (us a window with it / without: sorted arrays 1,024
 // LPs x 16 7.5 / 6.1, 20,000 x 30 25.6 / 21.3, 65,536 x 64 61.1 / 56.3; heaps 8,191 x 120
-// 32.2 / 30.2).
+// 32.2 / 30.2; time buckets 20,000 x 30 19.6 / 15.6, 65,536 x 64 30.3 / 27.4, where hashes
+// kept in shared memory and added up by two lanes an LP took 16.4 and 27.6).
 __device__ __forceinline__ void shared_add_u64(unsigned long long* p, uint64_t v) {
   uint32_t* w = reinterpret_cast<uint32_t*>(p);
   const uint32_t lo = (uint32_t)v, old = atomicAdd(&w[0], lo);
