@@ -114,13 +114,15 @@ inline uint32_t laq_lanes(const gpq_phold_config& c) {
 
 // Whether the local heap queue takes a warp per LP and a window's items in one piece
 // (lhqw_lp_stage) where no number of lanes is asked for: with many events per LP and
-// window, or while one wave of warps holds all LPs; otherwise the warp's fixed steps cost
-// more than a few single pops.  Measured (us a window, 8 lanes / warp; events per LP and
-// window): 1,024 LPs 21.6 / 9.6 (8), 3,000 12.2 / 11.2 (2), 6,000 13.1 / 18.3 (2), 8,191
-// 42.4 / 32.0 (11), 20,011 24.8 / 39.5 (2) and 64.4 / 54.2 (8), 44,123 228 / 130 (20), 65,536
-// 104 / 139 (6) and 117 / 113 (8).
+// window, or, while one wave of warps holds all LPs, from a number of events that grows with
+// the LPs on; otherwise the warp's fixed steps cost more than a few single pops.  Measured
+// (us a window, 8 lanes / warp; events per LP and window): 64 LPs 5.9 / 6.1 (0.3), 8.6 / 7.3
+// (1.5); 1,024 7.2 / 7.0 (0.7), 19.8 / 8.5 (8); 3,000 7.5 / 8.4 (0.7), 11.5 / 10.2 (2); 4,096
+// 9.5 / 10.5 (1.3), 14.6 / 12.8 (3); 8,191 39.9 / 29.6 (11); 20,011 24.8 / 39.5 (2) and 58.4 /
+// 39.3 (8); 44,123 230 / 121 (21); 65,536 104 / 139 (6) and 112 / 103 (8).
 inline bool lhq_warp(const gpq_phold_config& c) {
-  return c.num_lps <= 4096 || (double)c.events_per_lp * c.lookahead / (1.0 + c.lookahead) >= 7.5;
+  const double events = (double)c.events_per_lp * c.lookahead / (1.0 + c.lookahead);
+  return events >= 7.5 || (c.num_lps <= 4096 && events >= std::max(0.5, c.num_lps / 2048.0));
 }
 
 // Lanes per LP that a run uses: the asked-for number, or by the rules above.  `c` is the
