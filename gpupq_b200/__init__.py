@@ -699,7 +699,7 @@ class PholdSession:
     """Resident PHOLD runs (gpq_phold_session_*): admit, step, collect.
 
     bucketed=True keeps the LP space as time buckets (gpq_phold_session_create_bucketed,
-    `buckets` x `bucket_slots` keys per LP, 0 = 32 x 16) instead of sorted rings
+    `buckets` x `bucket_slots` keys per LP, 0 = 32 x 16) instead of rings
     (capacity, insert_capacity, lanes_per_lp)."""
 
     def __init__(self, max_lps, max_instances, capacity=256, insert_capacity=64, lanes_per_lp=8, bucketed=False,
@@ -832,7 +832,7 @@ def serve_stream(seed, rate, duration, astar_fraction=0.8):
 def serve(reqs, n, mode=SERVE_BATCHED, budget=0, realtime=True, astar_rounds=0, phold_windows=0, astar_share=0.0,
           phold_form=0, **astar_cfg):
     """Run gpq_serve_run; returns (responses, stats dict).  phold_form 0 keeps the PHOLD
-    runs in sorted rings, 1 in time buckets."""
+    runs in rings, 1 in time buckets."""
     c = ServeConfig()
     c.phold_form = phold_form
     c.hbm_budget = budget

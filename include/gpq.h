@@ -195,7 +195,8 @@ typedef struct gpq_phold_config {
   uint32_t block_threads;   /* CTA size (multiple of 32); 0 = tuned default */
   uint32_t ctas_per_sm;     /* persistent grid: CTAs per SM; 0 = occupancy maximum */
   uint32_t max_steps;       /* safety cap on windows; 0 = none */
-  uint32_t lanes_per_lp;    /* LAQ: lanes that work on one LP (4, 8, 16 or 32); 0 = tuned default */
+  uint32_t lanes_per_lp;    /* LAQ: lanes that work on one LP (4, 8, 16 or 32); 0 = by the LPs and the
+                               events of a window */
   uint32_t node_size;       /* HQ: items per heap node r, a power of two in [2, 2^22]: one CTA
                              * works a heap of nodes up to 1,024 items, the whole GPU (one
                              * cooperative launch) larger ones; 0 = the reference's 256 K
@@ -350,7 +351,7 @@ typedef struct gpq_astar_config {
   uint32_t inbox_capacity;    /* items one tile receives per round; 0 = 8 * tile */
   uint32_t open_capacity;     /* items one tile keeps above the window; 0 = tile * tile */
   uint32_t frontier_capacity; /* shared-memory frontier items (two buffers); 0 = 2048 (256 per warp) */
-  uint32_t block_threads;     /* 64, 128 or 256; 0 = 256 */
+  uint32_t block_threads;     /* 64, 128 or 256; 0 = 512 where a block works a 64 x 64 tile, else 256 */
   uint32_t ctas_per_sm;       /* 0 = one per SM for every SM's worth of tiles expected active at a
                                  once (sqrt(tiles) per instance), at most as many as fit */
   uint32_t max_rounds;        /* 0 = 2^20; reaching it is GPQ_ERR_TIMEOUT */
@@ -453,18 +454,18 @@ GPQ_API gpq_status gpq_astar_query(uint64_t base_seed, uint32_t index, uint32_t 
  * together one window per grid barrier, each inside its own safe window
  * [min_i, min_i + lookahead_i), so each run commits exactly what it commits alone (same
  * committed count, steps, digest, pending events).  Finished runs are collected and give
- * their LPs back. */
+ * their LPs back.  lanes_per_lp (4, 8, 16 or 32; 0 = 8) bounds insert_capacity and is part of
+ * a snapshot's parameters; the windows' speed does not depend on it. */
 typedef struct gpq_phold_session gpq_phold_session;
 
 GPQ_API gpq_status gpq_phold_session_create(uint32_t max_lps, uint32_t capacity, uint32_t insert_capacity,
                                             uint32_t max_instances, uint32_t lanes_per_lp,
                                             gpq_phold_session** out);
-/* A session whose LP space holds time buckets instead of sorted rings (the bucketed local
+/* A session whose LP space holds time buckets instead of rings (the bucketed local
  * array queue, gpq_phold_config.laq_mode 2): `buckets` buckets of `bucket_slots` keys per
  * LP (powers of two; 0 = 32 and 16) and spill lists of max(64, bucket_slots) keys.  An
  * admitted run gets a bucket width from its lookahead and events_per_lp; a run whose
- * lookahead needs more buckets is refused (GPQ_ERR_INVALID).  Same results as the sorted
- * form. */
+ * lookahead needs more buckets is refused (GPQ_ERR_INVALID).  Same results as the rings. */
 GPQ_API gpq_status gpq_phold_session_create_bucketed(uint32_t max_lps, uint32_t buckets, uint32_t bucket_slots,
                                                      uint32_t max_instances, gpq_phold_session** out);
 GPQ_API gpq_status gpq_phold_session_destroy(gpq_phold_session* s);
@@ -535,8 +536,8 @@ typedef struct gpq_serve_config {
   gpq_astar_config astar;
   uint32_t phold_capacity;        /* per-LP queue capacity; 0 = 256 */
   uint32_t phold_insert_capacity; /* per-LP children per window; 0 = 64 */
-  uint32_t phold_lanes_per_lp;    /* sorted form: lanes per LP; 0 = 8 */
-  uint32_t phold_form;            /* 0 = sorted rings, 1 = time buckets (gpq_phold_session_create_bucketed) */
+  uint32_t phold_lanes_per_lp;    /* rings: checked and recorded (0 = 8), see gpq_phold_session_create */
+  uint32_t phold_form;            /* 0 = rings, 1 = time buckets (gpq_phold_session_create_bucketed) */
   uint32_t reserved[4];
 } gpq_serve_config;
 
