@@ -1282,8 +1282,9 @@ static __global__ void astar_pred_kernel(AstarDev d, const uint32_t* list) {
 // warps hash and store the cells it recorded.  Windows are placed around the current cell
 // with most of their room on the side of the start, where the path is heading.  Two forms:
 //  - instances of at least kAstarPredBytesCells cells (long walks, few of them at a time)
-//    use the predecessor moves that astar_pred_kernel wrote for every expanded cell:
-//    128 x 128 windows of move bytes, one shared-memory byte per step;
+//    use the predecessor moves that astar_pred_kernel wrote for every expanded cell: staged
+//    as 128 x 128 windows that hold each cell's next place, so that a step of the walk is one
+//    dependent shared-memory load and nothing else;
 //  - smaller instances (many at a time, where a pass over every expanded cell would
 //    cost more than it saves) stage 64 x 64 windows of g values and blocked
 //    bits, and warp 0 finds each step: lane l tests the l-th neighbour in increasing
@@ -1292,11 +1293,12 @@ static constexpr uint32_t kPathThreads = 512;
 static constexpr uint32_t kPathWalkCap = 2048;
 static constexpr int kPathWinB = 128;                  // move-byte window side
 static constexpr int kPathRowWords = kPathWinB / 4 + 1;  // aligned words that cover 128 bytes
+static constexpr uint32_t kPathUnroll = 8;             // steps between two looks at where the walk is
 static constexpr int kPathWinC = 64;                   // g-value window side
 static constexpr int kPathHalo = kPathWinC + 2;         // plus the cells its moves reach
-static constexpr int kPathStageBytes = kPathHalo * kPathHalo * 5 > kPathWinB * kPathRowWords * 4
+static constexpr int kPathStageBytes = kPathHalo * kPathHalo * 5 > kPathWinB * kPathWinB * 2
                                            ? kPathHalo * kPathHalo * 5
-                                           : kPathWinB * kPathRowWords * 4;
+                                           : kPathWinB * kPathWinB * 2;
 
 // First column (row) of a window of side win around coordinate c on an axis of n cells,
 // with the start at coordinate s: 7/8 of the room towards the start.
@@ -1307,51 +1309,87 @@ __device__ __forceinline__ int astar_path_origin(int c, int s, int n, int win) {
 }
 
 struct AstarPathSmem {
-  uint32_t* walk;  // [kPathWalkCap] cells recorded in the current window
-  uint32_t* cur;   // next cell to record
+  uint32_t* walk;    // [kPathWalkCap] cells recorded in the current window (move-byte form: entries' offsets)
+  uint32_t* cur;     // next cell to record
+  uint32_t* origin;  // move-byte form: the window's first cell
   uint32_t* nwalk;
   uint32_t* done;  // 0 walking, 1 reached the start, 2 no predecessor
 };
 
-// One window of the move-byte form: stage, then thread 0 walks.  Ends with a barrier.
-__device__ __forceinline__ void astar_path_window_bytes(const AstarDev& d, const AstarInstDev& I, uint32_t* s_pw,
+// One window of the move-byte form.  Staged: for each cell the byte offset of its
+// predecessor's entry; a cell whose walk ends here (the start, no predecessor, a predecessor
+// outside the window) points at itself, so the walk needs no test but now and then whether it
+// still moves.  Thread 0 then follows the offsets, and a cell of the border that the walk
+// cannot leave is the first one of the next window, which lies around it: only the start and
+// a cell without a predecessor stop the walk elsewhere.  A 2048^2 grid's 4,095 steps took
+// 0.40 ms when a step read a move byte, updated the coordinates and tested them, and take
+// 0.23 so.  Ends with a barrier.
+__device__ __forceinline__ void astar_path_window_bytes(const AstarDev& d, const AstarInstDev& I, uint16_t* s_next,
                                                         const AstarPathSmem& sm) {
-  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t tid = threadIdx.x;
   const int w = (int)I.g.width, h = (int)I.g.height;
   const uint32_t start = I.g.start, cur = *sm.cur;
+  const int sx = (int)(start % (uint32_t)w), sy = (int)(start / (uint32_t)w);
   const int cx = (int)(cur % (uint32_t)w), cy = (int)(cur / (uint32_t)w);
-  const int tx0 = astar_path_origin(cx, (int)(start % (uint32_t)w), w, kPathWinB);
-  const int ty0 = astar_path_origin(cy, (int)(start / (uint32_t)w), h, kPathWinB);
+  const int tx0 = astar_path_origin(cx, sx, w, kPathWinB);
+  const int ty0 = astar_path_origin(cy, sy, h, kPathWinB);
   const uint32_t* PW = reinterpret_cast<const uint32_t*>(d.pred);
-  const int rows = min(kPathWinB, h - ty0);
-  for (int r = (int)warp; r < rows; r += (int)(kPathThreads / 32)) {  // row r: its bytes from (tx0, ty0 + r) on
-    const uint64_t w0 = (I.cell0 + (uint64_t)(ty0 + r) * (uint64_t)w + (uint64_t)tx0) >> 2;
-    const uint32_t a = __ldg(&PW[w0 + lane]);
-    const uint32_t b = lane == 0 ? __ldg(&PW[w0 + 32]) : 0u;
-    s_pw[r * kPathRowWords + (int)lane] = a;
-    if (lane == 0) s_pw[r * kPathRowWords + 32] = b;
+  const int cols = min(kPathWinB, w - tx0), rows = min(kPathWinB, h - ty0);
+  // words of four moves, a thread's loads in flight together
+  constexpr int kWords = kPathWinB * kPathRowWords, kEach = (kWords + (int)kPathThreads - 1) / (int)kPathThreads;
+  uint32_t mv[kEach];
+#pragma unroll
+  for (int u = 0; u < kEach; ++u) {
+    const int k = u * (int)kPathThreads + (int)tid, r = k / kPathRowWords, j = k % kPathRowWords;
+    mv[u] = 0u;
+    if (r < rows) {
+      const uint64_t b0 = I.cell0 + (uint64_t)(ty0 + r) * (uint64_t)w + (uint64_t)tx0;
+      if ((int)(4 * j) - (int)(b0 & 3u) < cols) mv[u] = __ldg(&PW[(b0 >> 2) + (uint32_t)j]);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kEach; ++u) {
+    const int k = u * (int)kPathThreads + (int)tid, r = k / kPathRowWords, j = k % kPathRowWords;
+    if (r >= rows) continue;
+    const int x0 = 4 * j - (int)((I.cell0 + (uint64_t)(ty0 + r) * (uint64_t)w + (uint64_t)tx0) & 3u);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const int x = x0 + t;
+      if (x < 0 || x >= cols) continue;
+      const uint32_t m = (mv[u] >> (8 * t)) & 0xffu;
+      const int nx = x + (int)(m & 3u) - 1, ny = r + (int)(m >> 2) - 1;
+      const bool stop = m == kAstarNoPred || nx < 0 || ny < 0 || nx >= cols || ny >= rows ||
+                        (tx0 + x == sx && ty0 + r == sy);
+      s_next[r * kPathWinB + x] = (uint16_t)(2 * (stop ? r * kPathWinB + x : ny * kPathWinB + nx));
+    }
   }
   __syncthreads();
   if (tid == 0) {
-    const uint8_t* s_pb = reinterpret_cast<const uint8_t*>(s_pw);
-    uint32_t c = cur, q = 0, done = 0;
-    uint32_t pc = (uint32_t)(I.cell0 + cur);  // its low two bits give each row's offset in its words
-    int lx = cx - tx0, ly = cy - ty0;
-    while (lx >= 0 && ly >= 0 && lx < kPathWinB && ly < kPathWinB && q < kPathWalkCap) {
-      sm.walk[q++] = c;
-      if (c == start) { done = 1; break; }
-      const uint32_t mv = s_pb[ly * (kPathRowWords * 4) + lx + (int)((pc - (uint32_t)lx) & 3u)];
-      if (mv == kAstarNoPred) { done = 2; break; }
-      const int dx = (int)(mv & 3u) - 1, dy = (int)(mv >> 2) - 1;
-      lx += dx;
-      ly += dy;
-      const uint32_t step = (uint32_t)(dy * w + dx);  // modulo 2^32: a step back is a wrapped add
-      c += step;
-      pc += step;
+    const unsigned char* nb = reinterpret_cast<const unsigned char*>(s_next);
+    uint32_t at = 2u * (uint32_t)((cy - ty0) * kPathWinB + (cx - tx0)), before = at, q = 0;
+    do {
+#pragma unroll
+      for (uint32_t u = 0; u < kPathUnroll; ++u) {
+        sm.walk[q + u] = at;
+        before = at;
+        at = *reinterpret_cast<const uint16_t*>(nb + at);
+      }
+      q += kPathUnroll;
+    } while (at != before && q + kPathUnroll <= kPathWalkCap);
+    uint32_t done = 0;
+    const int lx = (int)((at >> 1) % (uint32_t)kPathWinB), ly = (int)((at >> 1) / (uint32_t)kPathWinB);
+    const uint32_t c = (uint32_t)(ty0 + ly) * (uint32_t)w + (uint32_t)(tx0 + lx);
+    if (at == before) {  // it stays at c: once is enough, and not at all if the next window goes on from it
+      while (q > 0 && sm.walk[q - 1] == at) --q;
+      const bool edge = lx == 0 || ly == 0 || lx == cols - 1 || ly == rows - 1;
+      if (c == start) done = 1;
+      else if (!edge || q == 0) done = 2;  // a window lies around its first cell: it could have left
+      if (done) sm.walk[q++] = at;
     }
     *sm.cur = c;
     *sm.nwalk = q;
     *sm.done = done;
+    *sm.origin = (uint32_t)ty0 * (uint32_t)w + (uint32_t)tx0;
   }
   __syncthreads();
 }
@@ -1444,7 +1482,7 @@ static __global__ void __launch_bounds__(kPathThreads) astar_path_kernel(AstarDe
                                                                          uint32_t* path, uint32_t cap) {
   __shared__ __align__(16) uint8_t s_stage[kPathStageBytes];
   __shared__ uint32_t s_walk[kPathWalkCap];
-  __shared__ uint32_t s_cur, s_len, s_done, s_nwalk;
+  __shared__ uint32_t s_cur, s_len, s_done, s_nwalk, s_origin;
   __shared__ unsigned long long s_hs;
   const uint32_t j = blockIdx.x;
   if (j >= n) return;
@@ -1456,7 +1494,7 @@ static __global__ void __launch_bounds__(kPathThreads) astar_path_kernel(AstarDe
     return;
   }
   const bool bytes = astar_pred_bytes(I);
-  const AstarPathSmem sm{s_walk, &s_cur, &s_nwalk, &s_done};
+  const AstarPathSmem sm{s_walk, &s_cur, &s_origin, &s_nwalk, &s_done};
   const uint64_t cells = (uint64_t)I.g.width * I.g.height;
   if (tid == 0) {
     s_cur = I.g.goal;
@@ -1468,13 +1506,14 @@ static __global__ void __launch_bounds__(kPathThreads) astar_path_kernel(AstarDe
   // every window records at least one cell: at most cells + 1 windows
   for (uint64_t it = 0; it <= cells && s_done == 0u; ++it) {
     if (bytes)
-      astar_path_window_bytes(d, I, reinterpret_cast<uint32_t*>(s_stage), sm);
+      astar_path_window_bytes(d, I, reinterpret_cast<uint16_t*>(s_stage), sm);
     else
       astar_path_window_cells(d, I, reinterpret_cast<uint32_t*>(s_stage), s_stage + kPathHalo * kPathHalo * 4, sm);
     const uint32_t nw = s_nwalk, len0 = s_len;
     unsigned long long part = 0;
     for (uint32_t q = tid; q < nw; q += kPathThreads) {
-      const uint32_t c = s_walk[q];
+      uint32_t c = s_walk[q];
+      if (bytes) c = s_origin + (c >> 1) / (uint32_t)kPathWinB * I.g.width + (c >> 1) % (uint32_t)kPathWinB;
       part += gpq_astar_path_hash(len0 + q, c);
       if (path && i == want && len0 + q < cap) path[len0 + q] = c;
     }

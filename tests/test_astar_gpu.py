@@ -187,6 +187,22 @@ def test_path_forms(gpu_lib):
             assert int(r[k]) == want[i][k], (i, k)
 
 
+@pytest.mark.parametrize("w,h,dens,conn,start,goal", [
+    (100, 10487, 0.1, 8, 3, 100 * 10486 + 50),          # narrower than a window of the walk
+    (10487, 101, 0.1, 4, 10487 * 100 + 9, 10400),       # lower than one
+    (1027, 1029, 0.38, 8, 1027 * 500 + 500, 1027 * 510 + 530),  # winding, both ends inside
+    (1027, 1029, 0.33, 4, 1027 * 1028 + 1026, 2),       # winding, towards the larger ids
+    (1024, 1025, 0.2, 4, 70000, 70000), (1024, 1025, 0.0, 8, 70000, 70001),  # no step, one step
+])
+def test_move_byte_paths(gpu_lib, w, h, dens, conn, start, goal):
+    g = G.astar_grid(w, h, dens, 31, conn=conn, start=start, goal=goal)
+    want = O.astar({k: int(g[0][k]) for k in O.ASTAR_FIELDS}, want_path=True)
+    with G.AStar(tile=64) as a:
+        _check(a.solve(g), g)
+        if want["cost"] != G.ASTAR_INF:
+            assert np.array_equal(a.path(0), want["path"])
+
+
 def test_autotune_astar(gpu_lib, tmp_path):
     """The A* tuner times its candidates on the batch and returns one whose results are exact."""
     from gpupq_b200 import autotune
