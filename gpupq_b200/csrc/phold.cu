@@ -162,6 +162,69 @@ gpq_phold_params params_of(const gpq_phold_config& c) { return gpq::phold_params
 
 gpq_status validate(const gpq_phold_config* c) { return gpq::validate_phold_config(c); }
 
+// Heap nodes: the buffers whose size depends on the node size r (N items in all).
+std::vector<void**> hq_layout_buffers(HqDev* q, HqgDev* g) {
+  return {(void**)&q->nodes, (void**)&q->cnt,  (void**)&g->root2, (void**)&g->t0,    (void**)&g->t1,
+          (void**)&g->pa,    (void**)&g->pb,   (void**)&g->bref,  (void**)&g->k0,    (void**)&g->k1,
+          (void**)&g->rank,  (void**)&g->addc, (void**)&g->ilist, (void**)&g->icnt,  (void**)&g->plist,
+          (void**)&g->pcnt};
+}
+
+uint32_t hq_max_nodes(uint64_t N, uint32_t r) { return (uint32_t)((N + r - 1) / r + 2); }
+
+void hq_free_layout(HqDev* q, HqgDev* g) {
+  for (void** p : hq_layout_buffers(q, g)) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
+}
+
+// Allocates them into *q and *g (other fields as they were); on an error nothing is held.
+cudaError_t hq_alloc_layout(uint64_t N, uint32_t r, bool grid, HqDev* q, HqgDev* g) {
+  for (void** p : hq_layout_buffers(q, g)) *p = nullptr;
+  q->r = r;
+  q->maxnodes = hq_max_nodes(N, r);
+  cudaError_t e = cudaMalloc(&q->nodes, (size_t)q->maxnodes * r * sizeof(gpq_item));
+  auto get = [&](auto** p, size_t n) {
+    if (e == cudaSuccess) e = cudaMalloc(p, n);
+  };
+  get(&q->cnt, (size_t)q->maxnodes * sizeof(uint32_t));
+  if (grid) {
+    get(&g->root2, (size_t)r * sizeof(gpq_item));
+    get(&g->t0, (size_t)2 * r * sizeof(gpq_item));
+    get(&g->t1, (size_t)3 * r * sizeof(gpq_item));
+    get(&g->pa, (size_t)r * sizeof(gpq_item));
+    get(&g->pb, (size_t)r * sizeof(gpq_item));
+    get(&g->bref, (size_t)r * sizeof(gpq_item));
+    get(&g->k0, (size_t)r * sizeof(unsigned long long));
+    get(&g->k1, (size_t)r * sizeof(unsigned long long));
+    get(&g->rank, (size_t)r * sizeof(uint32_t));
+    get(&g->addc, (size_t)r * sizeof(uint32_t));
+    if (N <= r) {  // the root holds every item: bucket lists
+      get(&g->ilist, (size_t)kHqgMaxBuckets * kHqgListCapI * sizeof(gpq_item));
+      get(&g->icnt, 2 * kHqgMaxBuckets * sizeof(uint32_t));
+      get(&g->plist, (size_t)kHqgMaxBuckets * kHqgListCapP * sizeof(unsigned long long));
+      get(&g->pcnt, 2 * kHqgMaxBuckets * sizeof(uint32_t));
+    }
+  }
+  if (e != cudaSuccess) hq_free_layout(q, g);
+  return e;
+}
+
+// Node size where none is asked for.  A root that holds the whole population (up to the
+// largest node) makes a window three phases over bucket lists instead of merges down the
+// heap.  Measured (us a window, 256 K nodes / one root): 265,000 items 184 / 30 (5 % of them
+// in a window) and 268 / 156 (90 %), 600,000 314 / 49 (33 %), 1.2 M 390 / 57 (20 %), 4.2 M
+// 242 / 57 (0.1 %), 751 / 97 (9 %), 4,947 / 2,237 (90 %).  Larger populations get the
+// reference's 256 K nodes, and so does a run that goes on from a snapshot with them.
+constexpr uint32_t kHqRefNode = 256u << 10;
+uint32_t hq_default_node(uint64_t N, uint32_t most) {
+  if (N > most) return kHqRefNode;
+  uint32_t r = 2048;
+  while (r < N) r <<= 1;
+  return r;
+}
+
 }  // namespace
 
 extern "C" {
@@ -204,13 +267,8 @@ gpq_status gpq_phold_create(const gpq_phold_config* cfg_in, gpq_phold** out) {
     return fail(GPQ_ERR_INVALID);
   }
   if (c.queue_kind == GPQ_QUEUE_HQ || gaq_array) {
-    // Default node size: the reference's 256 K root; a smaller population gets a root that
-    // just holds it (a larger root changes nothing but its buffers' size).
     uint32_t r = gaq_array ? 0u : c.node_size;
-    if (r == 0) {
-      r = 2048;
-      while (r < pop && r < (gaq_array ? kHqgMaxR : (256u << 10))) r <<= 1;
-    }
+    if (r == 0) r = hq_default_node(pop, kHqgMaxR);
     const bool grid = r > kHqMaxR;
     if (!gpq::is_pow2(r) || r < 2 || r > kHqgMaxR || (!grid && c.num_lps > (1u << 21))) {
       gpq::set_last_error("heap queue: node_size must be a power of two in [2, %u] (num_lps <= 2^21 up to node "
@@ -219,10 +277,12 @@ gpq_status gpq_phold_create(const gpq_phold_config* cfg_in, gpq_phold** out) {
     }
     const uint64_t N = (uint64_t)c.num_lps * c.events_per_lp;
     h->is_hq = true;
-    h->hq.r = r;
-    h->hq.maxnodes = (uint32_t)((N + r - 1) / r + 2);
-    TRY(cudaMalloc(&h->hq.nodes, (size_t)h->hq.maxnodes * r * sizeof(gpq_item)));
-    TRY(cudaMalloc(&h->hq.cnt, (size_t)h->hq.maxnodes * sizeof(uint32_t)));
+    cudaError_t le = hq_alloc_layout(N, r, grid, &h->hq, &h->hqg);
+    if (le == cudaErrorMemoryAllocation && !gaq_array && c.node_size == 0 && r > kHqRefNode) {  // the smaller layout
+      cudaGetLastError();
+      le = hq_alloc_layout(N, kHqRefNode, grid, &h->hq, &h->hqg);
+    }
+    TRY(le);
     TRY(cudaMalloc(&h->hq.meta, 4 * sizeof(uint32_t)));
     TRY(cudaMalloc(&h->hq_sort[0], N * sizeof(gpq_item)));
     TRY(cudaMalloc(&h->hq_sort[1], N * sizeof(gpq_item)));
@@ -232,23 +292,7 @@ gpq_status gpq_phold_create(const gpq_phold_config* cfg_in, gpq_phold** out) {
     if (grid) {
       HqgDev& g = h->hqg;
       h->hq_grid = true;
-      TRY(cudaMalloc(&g.root2, (size_t)r * sizeof(gpq_item)));
-      TRY(cudaMalloc(&g.t0, (size_t)2 * r * sizeof(gpq_item)));
-      TRY(cudaMalloc(&g.t1, (size_t)3 * r * sizeof(gpq_item)));
-      TRY(cudaMalloc(&g.pa, (size_t)r * sizeof(gpq_item)));
-      TRY(cudaMalloc(&g.pb, (size_t)r * sizeof(gpq_item)));
-      TRY(cudaMalloc(&g.bref, (size_t)r * sizeof(gpq_item)));
-      TRY(cudaMalloc(&g.k0, (size_t)r * sizeof(unsigned long long)));
-      TRY(cudaMalloc(&g.k1, (size_t)r * sizeof(unsigned long long)));
-      TRY(cudaMalloc(&g.rank, (size_t)r * sizeof(uint32_t)));
-      TRY(cudaMalloc(&g.addc, (size_t)r * sizeof(uint32_t)));
       TRY(cudaMalloc(&g.ovf, sizeof(uint32_t)));
-      if ((uint64_t)c.num_lps * c.events_per_lp <= r) {  // the root holds every item: bucket lists
-        TRY(cudaMalloc(&g.ilist, (size_t)kHqgMaxBuckets * kHqgListCapI * sizeof(gpq_item)));
-        TRY(cudaMalloc(&g.icnt, 2 * kHqgMaxBuckets * sizeof(uint32_t)));
-        TRY(cudaMalloc(&g.plist, (size_t)kHqgMaxBuckets * kHqgListCapP * sizeof(unsigned long long)));
-        TRY(cudaMalloc(&g.pcnt, 2 * kHqgMaxBuckets * sizeof(uint32_t)));
-      }
       g.e2 = h->hq_sort[0];  // after populate: the sort scratch of a window's children
       TRY(gpq::raise_smem_limit(hqg_phold_kernel, hqg_smem_bytes()));
       int per_sm = 0;
@@ -786,18 +830,61 @@ gpq_status gpq_phold_restore(gpq_phold* h, const void* buf, uint64_t size, void*
   GPQ_CHECK_ARG(take(&cfg, sizeof(cfg)) && std::memcmp(&cfg, &h->cfg, sizeof(cfg)) == 0,
                 "snapshot of a run with another configuration");
   GPQ_CHECK_ARG(take(counts, 8) && counts[0] == dev.size() && counts[1] == host.size(), "snapshot layout differs");
+  // a heap of the default node size: the snapshot may hold the other of its two layouts
+  HqDev old_q{}, *swapped = nullptr;
+  HqgDev old_g{};
+  if (h->is_hq && h->hq_grid && h->cfg.queue_kind == GPQ_QUEUE_HQ && h->cfg.node_size == 0) {
+    const uint64_t N = (uint64_t)h->cfg.num_lps * h->cfg.events_per_lp;
+    const uint32_t one = hq_default_node(N, kHqgMaxR), other = h->hq.r == one ? std::min(one, kHqRefNode) : one;
+    const unsigned char* at = p;
+    for (size_t i = 0; i < dev.size() && (uint64_t)(end - at) >= 8; ++i) {
+      uint64_t n = 0;
+      std::memcpy(&n, at, 8);
+      if (dev[i].first == (void*)h->hq.nodes && other != h->hq.r &&
+          n == (uint64_t)hq_max_nodes(N, other) * other * sizeof(gpq_item)) {
+        old_q = h->hq;
+        old_g = h->hqg;
+        HqDev q = h->hq;
+        HqgDev g = h->hqg;
+        const cudaError_t e = hq_alloc_layout(N, other, true, &q, &g);
+        if (e != cudaSuccess) {
+          gpq::set_last_error("gpq_phold_restore: %s", cudaGetErrorString(e));
+          return e == cudaErrorMemoryAllocation ? GPQ_ERR_NOMEM : GPQ_ERR_CUDA;
+        }
+        h->hq = q;
+        h->hqg = g;
+        swapped = &old_q;
+        dev.clear();
+        host.clear();
+        phold_state(h, &dev, &host);
+        break;
+      }
+      if ((uint64_t)(end - at - 8) < n) break;
+      at += 8 + n;
+    }
+  }
+  auto refuse = [&](const char* why) {  // nothing has been overwritten: back to the handle's own layout
+    if (swapped) {
+      hq_free_layout(&h->hq, &h->hqg);
+      h->hq = old_q;
+      h->hqg = old_g;
+    }
+    gpq::set_last_error("invalid: %s", why);
+    return GPQ_ERR_INVALID;
+  };
   // check every region's size before anything is overwritten
   const unsigned char* scan = p;
   for (size_t i = 0; i < dev.size() + host.size(); ++i) {
     const size_t want = i < dev.size() ? dev[i].second : host[i - dev.size()].second;
     uint64_t n = 0;
-    GPQ_CHECK_ARG((uint64_t)(end - scan) >= 8, "snapshot truncated");
+    if ((uint64_t)(end - scan) < 8) return refuse("snapshot truncated");
     std::memcpy(&n, scan, 8);
-    GPQ_CHECK_ARG(n == want && (uint64_t)(end - scan - 8) >= n, "snapshot region differs or is truncated");
+    if (n != want || (uint64_t)(end - scan - 8) < n) return refuse("snapshot region differs or is truncated");
     scan += 8 + n;
   }
   const cudaStream_t st = gpq::as_stream(stream, h->own);
   GPQ_CUDA_TRY(cudaStreamSynchronize(st));
+  if (swapped) hq_free_layout(&old_q, &old_g);
   for (auto& r : dev) {
     p += 8;
     GPQ_CUDA_TRY(cudaMemcpyAsync(r.first, p, r.second, cudaMemcpyHostToDevice, st));

@@ -199,9 +199,9 @@ typedef struct gpq_phold_config {
                                events of a window */
   uint32_t node_size;       /* HQ: items per heap node r, a power of two in [2, 2^22]: one CTA
                              * works a heap of nodes up to 1,024 items, the whole GPU (one
-                             * cooperative launch) larger ones; 0 = the reference's 256 K
-                             * (HQ_NODE_SIZE, src/config.h:88), lowered to the population
-                             * rounded up to a power of two (at least 2,048) */
+                             * cooperative launch) larger ones; 0 = the population rounded up
+                             * to a power of two (at least 2,048), or the reference's 256 K
+                             * (HQ_NODE_SIZE, src/config.h:88) above 4 M items */
   uint32_t laq_mode;        /* LAQ: 0 = sorted runs, children merged each window; 1 = unordered
                                arrays, each window's safe events selected and ranked; 2 = time
                                buckets of 8-byte keys per LP, each window's buckets ranked

@@ -80,3 +80,37 @@ def test_bad_snapshots_are_refused(gpu_lib):
         with G.Phold(_cfg("laq", 2, seed=43)) as other:
             with pytest.raises(G.GpqError):
                 other.restore(snap)
+
+
+def test_heap_layouts_restore_into_each_other(gpu_lib):
+    """A heap of the default node size may hold a snapshot in 256 K nodes (of a library whose
+    default they were, or of a handle that had restored one) as well as its own single root."""
+    cfgd = dict(num_lps=10007, events_per_lp=30, lookahead=0.4, end_time=6.0, seed=3, dest_mode=1, ring_width=7)
+
+    def run(h):
+        h.run()
+        r, s = h.result(), h.lp_stats()
+        return {k: r[k] for k in ("committed", "steps", "pending", "pending_csum", "digest", "status_code")}, s["ohash"]
+
+    def snap(node_size):
+        with G.Phold(G.make_phold_config(**cfgd, queue="hq", node_size=node_size)) as h:
+            h.populate()
+            h.step(5)
+            return h.snapshot()
+
+    nodes, root = snap(1 << 18), snap(0)
+    at = 8 + G.PholdConfig.node_size.offset
+    nodes[at:at + 4] = 0  # as a handle of the default size writes it
+    assert len(nodes) != len(root)
+    with G.Phold(G.make_phold_config(**cfgd, queue="hq")) as h:
+        h.populate()
+        want = run(h)
+        assert want[0]["status_code"] == 0
+        with pytest.raises(G.GpqError):
+            h.restore(nodes[:-9])  # truncated: refused, the handle as it was
+        for b in (nodes, root, nodes, nodes):
+            h.restore(b)
+            got = run(h)
+            assert got[0] == want[0] and np.array_equal(got[1], want[1])
+        h.populate()
+        assert run(h)[0] == want[0]
