@@ -304,7 +304,19 @@ class GaqQueue final : public QueueImpl {
                      cudaStream_t st) override {
     *n_out = 0;
     if (n_ == 0) return GPQ_OK;
-    if (max_per_lp == 0 && emit_ctas() <= kEmitCtas) return dequeue_prefix(bound, out, out_capacity, n_out, st);
+    // the LPs' lists that a refused or failed dequeue left filled, emptied on this one's stream
+    if (lists_filled_) GPQ_CUDA_TRY(cudaMemsetAsync(cnt_, 0, (size_t)L_ * sizeof(uint32_t), st));
+    lists_filled_ = true;
+    const gpq_status s = max_per_lp == 0 && emit_ctas() <= kEmitCtas
+                             ? dequeue_prefix(bound, out, out_capacity, n_out, st)
+                             : dequeue_limited(bound, max_per_lp, out, out_capacity, n_out, st);
+    if (s == GPQ_OK) lists_filled_ = false;  // gq_emit_kernel and gq_take_kernel empty them
+    else cudaStreamSynchronize(st);          // nothing of it runs on when it returns
+    return s;
+  }
+
+  gpq_status dequeue_limited(float bound, uint32_t max_per_lp, gpq_item* out, uint64_t out_capacity, uint64_t* n_out,
+                             cudaStream_t st) {
     const gpq_item* a = base();
     gaq_split_kernel<<<1, 32, 0, st>>>(a, n_, bound, 3.0e38f, words_);
     GPQ_CUDA_TRY(cudaMemcpyAsync(h_words_, words_, 4, cudaMemcpyDeviceToHost, st));
@@ -360,10 +372,9 @@ class GaqQueue final : public QueueImpl {
     GPQ_CUDA_TRY(cudaMemcpyAsync(h_words_, words_, 9 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     GPQ_CUDA_TRY(cudaStreamSynchronize(st));
     const uint32_t c = h_words_[0], e = h_words_[8];
-    if (!e) *n_out = c;
-    if (e || c > out_capacity) {
-      GPQ_CUDA_TRY(cudaMemsetAsync(cnt_, 0, (size_t)L_ * sizeof(uint32_t), st));
-      if (e) return (gpq_status)e;
+    if (e) return (gpq_status)e;
+    *n_out = c;
+    if (c > out_capacity) {
       set_last_error("dequeue: %u items do not fit the output", c);
       return GPQ_ERR_INVALID;
     }
@@ -441,6 +452,7 @@ class GaqQueue final : public QueueImpl {
   int cur_ = 0;
   uint32_t head_ = 0;  // the array's items are arr_[cur_][head_, head_ + n_)
   const gpq_item* base() const { return arr_[cur_] + head_; }
+  bool lists_filled_ = false;  // cnt_ may be other than zero
   uint32_t emit_ctas() const { return (L_ + kEmitLps - 1) / kEmitLps; }
   uint32_t* sums_ = nullptr;  // [emit_ctas()]
   struct Host {               // page-locked
