@@ -179,7 +179,8 @@ void hq_free_layout(HqDev* q, HqgDev* g) {
   }
 }
 
-// Allocates them into *q and *g (other fields as they were); on an error nothing is held.
+// Allocates them into *q and *g (other fields as they were).  On an error nothing is held, and
+// the runtime's last error is cleared: a caller that goes on must not find it at its next launch.
 cudaError_t hq_alloc_layout(uint64_t N, uint32_t r, bool grid, HqDev* q, HqgDev* g) {
   for (void** p : hq_layout_buffers(q, g)) *p = nullptr;
   q->r = r;
@@ -207,7 +208,10 @@ cudaError_t hq_alloc_layout(uint64_t N, uint32_t r, bool grid, HqDev* q, HqgDev*
       get(&g->pcnt, 2 * kHqgMaxBuckets * sizeof(uint32_t));
     }
   }
-  if (e != cudaSuccess) hq_free_layout(q, g);
+  if (e != cudaSuccess) {
+    hq_free_layout(q, g);
+    cudaGetLastError();
+  }
   return e;
 }
 
@@ -278,10 +282,8 @@ gpq_status gpq_phold_create(const gpq_phold_config* cfg_in, gpq_phold** out) {
     const uint64_t N = (uint64_t)c.num_lps * c.events_per_lp;
     h->is_hq = true;
     cudaError_t le = hq_alloc_layout(N, r, grid, &h->hq, &h->hqg);
-    if (le == cudaErrorMemoryAllocation && !gaq_array && c.node_size == 0 && r > kHqRefNode) {  // the smaller layout
-      cudaGetLastError();
+    if (le == cudaErrorMemoryAllocation && !gaq_array && c.node_size == 0 && r > kHqRefNode)  // the smaller layout
       le = hq_alloc_layout(N, kHqRefNode, grid, &h->hq, &h->hqg);
-    }
     TRY(le);
     TRY(cudaMalloc(&h->hq.meta, 4 * sizeof(uint32_t)));
     TRY(cudaMalloc(&h->hq_sort[0], N * sizeof(gpq_item)));
