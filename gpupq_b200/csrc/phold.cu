@@ -233,9 +233,8 @@ uint32_t hq_default_node(uint64_t N, uint32_t most) {
 
 extern "C" {
 
-gpq_status gpq_phold_create(const gpq_phold_config* cfg_in, gpq_phold** out) {
-  GPQ_CHECK_ARG(out, "out is NULL");
-  *out = nullptr;
+// ref_nodes: a heap of the default node size takes 256 K nodes whatever its population.
+static gpq_status create_handle(const gpq_phold_config* cfg_in, bool ref_nodes, gpq_phold** out) {
   gpq_status st = validate(cfg_in);
   if (st != GPQ_OK) return st;
   gpq_phold_config c = *cfg_in;
@@ -272,7 +271,7 @@ gpq_status gpq_phold_create(const gpq_phold_config* cfg_in, gpq_phold** out) {
   }
   if (c.queue_kind == GPQ_QUEUE_HQ || gaq_array) {
     uint32_t r = gaq_array ? 0u : c.node_size;
-    if (r == 0) r = hq_default_node(pop, kHqgMaxR);
+    if (r == 0) r = hq_default_node(pop, ref_nodes ? kHqRefNode : kHqgMaxR);
     const bool grid = r > kHqMaxR;
     if (!gpq::is_pow2(r) || r < 2 || r > kHqgMaxR || (!grid && c.num_lps > (1u << 21))) {
       gpq::set_last_error("heap queue: node_size must be a power of two in [2, %u] (num_lps <= 2^21 up to node "
@@ -281,10 +280,7 @@ gpq_status gpq_phold_create(const gpq_phold_config* cfg_in, gpq_phold** out) {
     }
     const uint64_t N = (uint64_t)c.num_lps * c.events_per_lp;
     h->is_hq = true;
-    cudaError_t le = hq_alloc_layout(N, r, grid, &h->hq, &h->hqg);
-    if (le == cudaErrorMemoryAllocation && !gaq_array && c.node_size == 0 && r > kHqRefNode)  // the smaller layout
-      le = hq_alloc_layout(N, kHqRefNode, grid, &h->hq, &h->hqg);
-    TRY(le);
+    TRY(hq_alloc_layout(N, r, grid, &h->hq, &h->hqg));
     TRY(cudaMalloc(&h->hq.meta, 4 * sizeof(uint32_t)));
     TRY(cudaMalloc(&h->hq_sort[0], N * sizeof(gpq_item)));
     TRY(cudaMalloc(&h->hq_sort[1], N * sizeof(gpq_item)));
@@ -383,6 +379,17 @@ gpq_status gpq_phold_create(const gpq_phold_config* cfg_in, gpq_phold** out) {
 #undef TRY
   *out = h;
   return GPQ_OK;
+}
+
+gpq_status gpq_phold_create(const gpq_phold_config* cfg, gpq_phold** out) {
+  GPQ_CHECK_ARG(out, "out is NULL");
+  *out = nullptr;
+  const gpq_status st = create_handle(cfg, false, out);
+  if (st != GPQ_ERR_NOMEM || cfg->queue_kind != GPQ_QUEUE_HQ || cfg->node_size != 0) return st;
+  const uint64_t pop = (uint64_t)cfg->num_lps * cfg->events_per_lp;
+  if (pop <= kHqRefNode || pop > kHqgMaxR) return st;
+  cudaGetLastError();  // one root and the rest of the handle do not fit: the smaller layout
+  return create_handle(cfg, true, out);
 }
 
 gpq_status gpq_phold_destroy(gpq_phold* h) {
