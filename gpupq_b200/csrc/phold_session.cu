@@ -226,10 +226,15 @@ std::vector<std::pair<void*, size_t>> session_regions(const gpq_phold_session* s
   return r;
 }
 
+// The header's last word: 1 for time buckets, and for rings whose events are sorted (which the
+// windows of earlier builds need and wrote); 2 for rings in any order.
+constexpr uint32_t kSessionSnapSorted = 1u, kSessionSnapRings = 2u;
+
 void session_header(const gpq_phold_session* s, uint32_t h[kSessionSnapHeader]) {
   const uint32_t v[kSessionSnapHeader] = {s->bucketed ? 1u : 0u, s->max_lps, s->max_inst, s->cap_log2, s->ibc,
                                           s->group, s->block, s->b.q.nb_log2, s->b.q.c_log2, s->b.q.F,
-                                          (uint32_t)sizeof(PmInstDev), 1u};
+                                          (uint32_t)sizeof(PmInstDev),
+                                          s->bucketed ? kSessionSnapSorted : kSessionSnapRings};
   std::memcpy(h, v, sizeof(v));
 }
 
@@ -315,7 +320,9 @@ gpq_status gpq_phold_session_restore(gpq_phold_session* s, const void* buf, uint
   uint32_t hdr[kSessionSnapHeader], mine[kSessionSnapHeader];
   session_header(s, mine);
   GPQ_CHECK_ARG(take(&magic, 8) && magic == kSessionSnapMagic, "not a PHOLD session snapshot");
-  GPQ_CHECK_ARG(take(hdr, sizeof(hdr)) && std::memcmp(hdr, mine, sizeof(hdr)) == 0,
+  const bool whole = take(hdr, sizeof(hdr));
+  if (whole && hdr[kSessionSnapHeader - 1] == kSessionSnapSorted) mine[kSessionSnapHeader - 1] = kSessionSnapSorted;
+  GPQ_CHECK_ARG(whole && std::memcmp(hdr, mine, sizeof(hdr)) == 0,
                 "snapshot of a session with other parameters");
   // host state into temporaries; nothing changes until every part has been checked
   uint64_t nb = 0;
