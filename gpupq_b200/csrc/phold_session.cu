@@ -661,7 +661,7 @@ uint64_t gpq_phold_session_bytes(uint32_t max_lps, uint32_t capacity, uint32_t i
                                  uint32_t max_instances) {
   if (capacity == 0) capacity = 256;
   if (insert_capacity == 0) insert_capacity = 64;
-  const uint64_t per_lp = 16ull * capacity + 32ull * insert_capacity + 4 * 6 + 8 * 2;
+  const uint64_t per_lp = 16ull * capacity + 32ull * insert_capacity + 4 * 7 + 8 * 2;
   return per_lp * max_lps + (uint64_t)max_instances * (sizeof(PmInstDev) + 24 + 1 + 4 + sizeof(PmAcc));
 }
 

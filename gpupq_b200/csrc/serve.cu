@@ -62,7 +62,7 @@ gpq_status serve_batched(const gpq_serve_config& c, const gpq_serve_request* req
   const uint32_t ibc = c.phold_insert_capacity ? c.phold_insert_capacity : 64;
   const uint64_t p_bytes = budget - std::min(budget, a_bytes);
   const bool buckets = c.phold_form == 1;
-  const uint64_t per_lp = buckets ? gpq_phold_session_bytes_bucketed(1, 0, 0, 0) : 16ull * cap + 32ull * ibc + 40;
+  const uint64_t per_lp = buckets ? gpq_phold_session_bytes_bucketed(1, 0, 0, 0) : gpq_phold_session_bytes(1, cap, ibc, 0);
   const uint32_t max_lps = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(p_bytes / per_lp, 1024), 1u << 30);
   Sessions ss;
   gpq_status st = gpq_astar_session_create(&ac, max_cells, max_tiles, max_inst, &ss.astar);
