@@ -863,16 +863,18 @@ __device__ void astar_process_tile(const AstarDev& d, uint32_t t, uint32_t s, As
     for (uint32_t j = wk.tid; j < (ts + 2u) * astar_sweep_stride(ts) / 8u; j += wk.n) vs4[j] = none;
     if (wk.tid < 3u) sm.moved[wk.tid] = 0;
   }
-  // (sixteen loads of a thread in flight at a time: the copy is a round trip to L2 otherwise repeated)
-  for (uint32_t l0 = wk.tid; l0 < ts * ts; l0 += 16u * wk.n) {
-    uint32_t g[16];
+  // Several loads of a thread in flight at a time: the copy is a round trip to L2 otherwise
+  // repeated.  Fewer where a CTA walks lists, which has 64 registers a thread.
+  constexpr uint32_t kFlight = sweeps || WARP ? 16u : 4u;
+  for (uint32_t l0 = wk.tid; l0 < ts * ts; l0 += kFlight * wk.n) {
+    uint32_t g[kFlight];
 #pragma unroll
-    for (uint32_t q = 0; q < 16; ++q) {
+    for (uint32_t q = 0; q < kFlight; ++q) {
       const uint32_t l = l0 + q * wk.n, lx = l & (ts - 1u), ly = l >> tg.lts;
       g[q] = (l < ts * ts && lx < tg.tw && ly < tg.th) ? ldcg_u32(&G[(tg.y0 + ly) * I.g.width + tg.x0 + lx]) : kAstarInf;
     }
 #pragma unroll
-    for (uint32_t q = 0; q < 16; ++q)
+    for (uint32_t q = 0; q < kFlight; ++q)
       if (l0 + q * wk.n < ts * ts) sm.gt[l0 + q * wk.n] = g[q];
   }
   wk.sync();
@@ -1028,9 +1030,13 @@ __host__ __device__ inline size_t astar_worker_smem_bytes(uint32_t ts, uint32_t 
 // (0 = no limit): a resident session resumes at the next round in its next launch.
 // NP: pairs of cells of a thread that sweeps (astar_sweep_pairs), 0: list walk.  With four
 // pairs one CTA of 512 threads an SM: a second would halve the registers and spill (2048 x
-// 2048 search 1.97 against 2.25 ms, 500 mixed searches 3.16 against 3.29 ms).
+// 2048 search 1.97 against 2.25 ms, 500 mixed searches 3.16 against 3.29 ms).  CTAs that
+// walk lists stay four an SM at 256 threads, since the visits of many searches hide each other's
+// chains (at two, with 104 registers: 500 mixed searches in tiles of 16 16.6 against 12.4 ms,
+// 2,000 small ones 4.9 / 3.9, in tiles of 8 33 / 21 and 8.6 / 5.8); warps that walk lists gain
+// more from loads in flight (tiles of 16: 19.4 ms, 20.5 at four).
 template <bool WARP, int NP>
-static __global__ void __launch_bounds__(NP == 4 ? 512 : 256, NP == 4 ? 1 : 2) astar_persistent_kernel(AstarDev d, uint32_t s0, uint32_t step_rounds) {
+static __global__ void __launch_bounds__(NP == 4 ? 512 : 256, NP == 4 ? 1 : NP == 8 || WARP ? 2 : 4) astar_persistent_kernel(AstarDev d, uint32_t s0, uint32_t step_rounds) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ AstarTileSmem sms[kAstarMaxWorkers];
   __shared__ uint32_t s_t;
