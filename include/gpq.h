@@ -351,7 +351,7 @@ typedef struct gpq_astar_config {
   uint32_t inbox_capacity;    /* items one tile receives per round; 0 = 8 * tile */
   uint32_t open_capacity;     /* items one tile keeps above the window; 0 = tile * tile */
   uint32_t frontier_capacity; /* shared-memory frontier items (two buffers); 0 = 2048 (256 per warp) */
-  uint32_t block_threads;     /* 64, 128 or 256; 0 = 512 where a block works a 64 x 64 tile, else 256 */
+  uint32_t block_threads;     /* 64, 128 or 256, or 512 where a block works a 64 x 64 tile; 0 = the largest */
   uint32_t ctas_per_sm;       /* 0 = one per SM for every SM's worth of tiles expected active at a
                                  once (sqrt(tiles) per instance), at most as many as fit */
   uint32_t max_rounds;        /* 0 = 2^20; reaching it is GPQ_ERR_TIMEOUT */
