@@ -94,22 +94,27 @@ inline uint32_t lsq_lanes(uint32_t num_lps) {
   return 1;
 }
 
-// Default lanes per LP of the sorted local array queue (laq_mode 0 and 1).  A wave of CTAs
-// holds 14,208 LPs with 8 lanes each, 7,104 with 16, 3,552 with 32.  In one wave a window is
-// one LP's chain of dependent steps, which more lanes shorten when the LP has several
+// Default lanes per LP of the local array queue, sorted (laq_mode 0) and unordered (1).  A wave
+// of CTAs holds 14,208 LPs with 8 lanes each, 7,104 with 16, 3,552 with 32.  In one wave a
+// window is one LP's chain of dependent steps, which more lanes shorten when the LP has several
 // events; between one and one and a half waves of 8 lanes, three short rounds of 16 beat two
-// long ones; otherwise the fixed steps per LP count and 8 lanes cost least.  Measured (us a
-// window, 8 / 16 / 32 lanes; events per LP and window): 1,024 LPs 6.7 / 6.3 / 5.7 (0.4),
-// 12.1 / 9.0 / 7.6 (8); 3,000 7.3 / 7.2 / 7.2 (0.8), 12.8 / 9.7 / 9.1 (8); 7,000 8.2 / 8.8
-// (0.8), 10.7 / 9.6 (3), 17.1 / 12.5 (11); 7,500 17.3 / 18.6 (11); 21,000 16.6 / 17.0 (3),
-// 26.0 / 22.4 (6), 55.0 / 46.4 (21); 24,000 29.5 / 34.0 (11); 40,000 17.2 / 25.9 (0.8),
-// 44.1 / 50.4 (11); 65,536 70.4 / 79.1 (11).
+// long ones; otherwise the fixed steps per LP count and 8 lanes cost least.  Where 8 lanes hold
+// all LPs at once and 16 do, or nearly do, the unordered arrays, whose events take fewer steps,
+// are later to gain from 16.  Measured (us a window, 8 / 16 / 32 lanes; events per LP and
+// window), sorted: 1,024 LPs 6.7 / 6.2 / 5.6 (0.8), 10.1 / 7.5 / 6.1 (8); 3,000 6.9 / 6.8 / 7.0
+// (0.8), 10.7 / 8.2 / 7.8 (8); 7,000 7.8 / 8.4 (0.8), 9.0 / 8.6 (3), 20.1 / 13.5 (11); 7,500
+// 20.3 / 20.8 (11); 21,000 14.8 / 15.8 (3), 18.1 / 17.0 (5), 42.3 / 33.7 (21); 24,000 38.1 /
+// 37.0 (11); 40,000 16.8 / 25.1 (0.8), 31.1 / 33.1 (8); 65,536 49.9 / 51.7 (8).  Unordered:
+// 1,024 8.1 / 6.4 / 5.1 (0.8), 11.2 / 7.2 / 5.3 (8); 3,000 8.3 / 6.9 / 6.4 (0.8), 11.7 / 7.8 /
+// 6.8 (8); 4,096 9.3 / 7.6 (3); 7,000 9.9 / 11.4 (3), 12.7 / 12.9 (8), 24.5 / 21.9 (11); 18,000
+// 18.5 / 19.3 (5), 44.8 / 40.4 (11); 21,000 27.5 / 26.1 (8); 40,000 44.5 / 43.3 (8).
 inline uint32_t laq_lanes(const gpq_phold_config& c) {
   const uint32_t L = c.num_lps;
   const double events = (double)c.events_per_lp * c.lookahead / (1.0 + c.lookahead);
+  const bool unordered = c.laq_mode == 1;
   if (L <= 2048 || (L <= 3552 && events >= 5.0)) return 32;
-  if (L <= 4096 || (L <= 7104 && events >= 2.5)) return 16;
-  return L > 14208 && L <= 21312 && events >= 5.0 ? 16 : 8;
+  if (L <= 4096 || (L <= 7104 && events >= (unordered ? 8.0 : 2.5))) return 16;
+  return L > 14208 && L <= 21312 && events >= (unordered ? 8.0 : 5.0) ? 16 : 8;
 }
 
 // Whether the local heap queue takes a warp per LP and a window's items in one piece
