@@ -148,6 +148,18 @@ __device__ __forceinline__ void pm_sel_file(const PmDev& d, uint32_t s, uint32_t
   else pm_error(d, inst, s, GPQ_ERR_INSERT_FULL);
 }
 
+// The ranks of a turn's events when some keys of an LP are equal (from a snapshot that holds
+// such events, or ids that wrap around), by their place in the list.  All lanes of the warp.
+static __device__ __noinline__ void pm_sel_rank_equal(const unsigned long long* key, uint32_t* at, uint32_t total) {
+  for (uint32_t y = threadIdx.x & 31u; y < total; y += 32u) {
+    const uint32_t seg = (at[y] >> 8) & 0xffu, j = at[y] & 0xffu;
+    const unsigned long long kj = key[seg * kPmSelStride + j];
+    uint32_t r = at[y] >> 16;
+    for (uint32_t t = 0; t < j; ++t) r += key[seg * kPmSelStride + t] == kj ? 1u : 0u;
+    at[y] = (r << 16) | (seg << 8) | j;
+  }
+}
+
 // An LP with more safe events than its list holds, by the whole warp (keys: the lists'
 // space): its safe keys side by side, ranked and processed one per lane -- beyond kPmWideCap
 // of them, ranked by scanning the LP's items --, then the rest moved down in order.  All
@@ -188,10 +200,17 @@ static __device__ __forceinline__ void pm_select_wide(const PmDev& d, uint32_t s
   for (uint32_t i = lane; i < top; i += 32u) {
     unsigned long long key;
     uint32_t r = 0;
-    if (fit) {
+    if (fit) {  // equal keys by their place: those before the warp's 32 also count when equal
       key = keys[i];
+      const uint32_t b = i - lane, e = min(b + 32u, sc);
 #pragma unroll 4
-      for (uint32_t t = 0; t < sc; t += 2u) {
+      for (uint32_t t = 0; t < b; t += 2u) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(keys + t);
+        r += (a.x <= key ? 1u : 0u) + (a.y <= key ? 1u : 0u);
+      }
+      for (uint32_t t = b; t < e; ++t) r += keys[t] < key || (keys[t] == key && t < i) ? 1u : 0u;
+#pragma unroll 4
+      for (uint32_t t = b + 32u; t < sc; t += 2u) {
         const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(keys + t);
         r += (a.x < key ? 1u : 0u) + (a.y < key ? 1u : 0u);
       }
@@ -201,7 +220,8 @@ static __device__ __forceinline__ void pm_select_wide(const PmDev& d, uint32_t s
       key = gpq_lp_key(e);
       for (uint32_t j = 0; j < m; ++j) {
         const gpq_item o = item(j);
-        r += (o.ts < lim && gpq_lp_key(o) < key) ? 1u : 0u;
+        const unsigned long long ko = gpq_lp_key(o);
+        r += o.ts < lim && (ko < key || (ko == key && j < i)) ? 1u : 0u;
       }
     }
     uint64_t h, oh;
@@ -385,6 +405,7 @@ static __device__ __forceinline__ uint32_t pm_select_turns(const PmDev& d, uint3
     const uint32_t inst0 = __shfl_sync(GPQ_FULL_MASK, li, __ffs(act) - 1);
     const bool one = __all_sync(GPQ_FULL_MASK, li == ~0u || li == inst0);  // all of one run
     __syncwarp();
+    uint32_t ranks = 0;
     for (uint32_t y = lane; y < total; y += 32u) {  // rank
       uint32_t seg = 0;
 #pragma unroll
@@ -399,6 +420,11 @@ static __device__ __forceinline__ uint32_t pm_select_turns(const PmDev& d, uint3
         r += (a.x < kj ? 1u : 0u) + (a.y < kj ? 1u : 0u);
       }
       sm.at[y] = (r << 16) | (seg << 8) | j;
+      ranks += r;
+    }
+    {  // equal keys share a rank, which the ranks' sum tells
+      const uint32_t ns = lane < kPmSelLps ? sm.beg[lane + 1u] - sm.beg[lane] : 1u;
+      if (__reduce_add_sync(GPQ_FULL_MASK, ranks - ns * (ns - 1u) / 2u) != 0u) pm_sel_rank_equal(sm.key, sm.at, total);
     }
     __syncwarp();
     uint32_t cmin = kInfBits;
