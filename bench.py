@@ -510,7 +510,7 @@ def bench_astar_ref(G, O, args, peak):
 def bench_phold_batched(G, O, args, peak):
     """The PHOLD runs of the first second of the served stream (LPs log-uniform in
     [256, 65536], 32 events per LP, lookahead 0.5, end time 200), all in one launch of a
-    session whose LP space holds sorted rings (the default session form); the same batch in
+    session whose LP space holds rings (the default session form); the same batch in
     a time-bucket session and the plain path (each run alone through its own handle, both
     queue forms) beside it."""
     reqs, n = G.serve_stream(99, 2000.0, 1.0)
@@ -563,7 +563,7 @@ def bench_phold_batched(G, O, args, peak):
     achieved = ev * BYTES_PER_EVENT * args.steps / dt / 1e9
     return {"workload": f"phold_batched_{len(runs)}runs_lp256-65536_x32_T200", "metric": "PHOLD events/s (batched)",
             "value": ev * args.steps / dt, "unit": "events/s", "runs": len(runs), "lps": lps,
-            "ms_per_batch": 1e3 * dt / args.steps, "queue_form": "sorted rings",
+            "ms_per_batch": 1e3 * dt / args.steps, "queue_form": "rings",
             "time_bucket_session_value": ev0 * args.steps / dt0, "same_results_both_forms": same,
             "plain_value": pv, "plain_bucketed_value": plain[2][0], "plain_sorted_value": plain[0][0],
             "plain_device_value": pdv,
@@ -614,7 +614,7 @@ def bench_served(G, args, duration):
             "exact_scope": "every request of the timed stream against the same request alone (plain path)",
             "capacity_note": "the PHOLD share alone needs about 20 G events/s at 2,000 requests/s "
                              "(400 runs/s x ~11,800 LPs x 32 events x ~133 events per chain), above the "
-                             "batched engine's ~12.8 G events/s: the offered rate is beyond one GPU",
+                             "batched engine's ~17 G events/s: the offered rate is beyond one GPU",
             "held_rate": {"offered_rate": 600.0, "seconds": 2.0, "requests": hn, "bad_status": hbad,
                           "batched": r(hst),
                           "sustained": bool(hst["throughput"] >= 0.9 * hn / 2.0 and hst["p99"] < 0.5)},

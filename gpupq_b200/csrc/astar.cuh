@@ -12,10 +12,11 @@
 //     scanned; stale items (g above the cell's current g) are dropped, items above the
 //     instance's best goal cost UB are pruned, items with f <= bound join the CTA's
 //     frontier in shared memory and the rest stay in the open array.  The CTA then
-//     expands the frontier level by level: a child whose g improves (atomicMin on the
-//     cell's g) goes to the next frontier when it lies in the tile and in the window,
-//     to the tile's open array when above the window, or to the owning tile's inbox for
-//     the next round.
+//     relaxes the whole tile from them in sweeps (astar_sweep_tile), or -- other tile
+//     sides, small CTAs, warps -- expands the frontier level by level: a child whose g
+//     improves (atomicMin on the cell's g) goes to the next frontier when it lies in the
+//     tile and in the window, to the tile's open array when above the window, or to the
+//     owning tile's inbox for the next round.
 //   * phase W: an instance whose tiles sent nothing for the next round has drained its
 //     window; the window moves to [min f of its open arrays, + delta], or the instance
 //     is done when that minimum exceeds UB.  The CTA that makes the instance's last visit

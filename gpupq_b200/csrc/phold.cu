@@ -219,8 +219,11 @@ cudaError_t hq_alloc_layout(uint64_t N, uint32_t r, bool grid, HqDev* q, HqgDev*
 // largest node) makes a window three phases over bucket lists instead of merges down the
 // heap.  Measured (us a window, 256 K nodes / one root): 265,000 items 184 / 30 (5 % of them
 // in a window) and 268 / 156 (90 %), 600,000 314 / 49 (33 %), 1.2 M 390 / 57 (20 %), 4.2 M
-// 242 / 57 (0.1 %), 751 / 97 (9 %), 4,947 / 2,237 (90 %).  Larger populations get the
-// reference's 256 K nodes, and so does a run that goes on from a snapshot with them.
+// 242 / 57 (0.1 %), 751 / 97 (9 %), 4,947 / 2,237 (90 %).  What it costs is memory (the whole
+// handle, one root / 256 K nodes): 300,000 items 0.19 / 0.12 GB, 2.6 M 1.15 / 0.32, 4.2 M 1.20 /
+// 0.39; snapshots 0.08 / 0.07, 0.42 / 0.27, 0.47 / 0.35.  Larger populations get the
+// reference's 256 K nodes, and so do a handle that would not fit otherwise and a run that goes
+// on from a snapshot with them.
 constexpr uint32_t kHqRefNode = 256u << 10;
 uint32_t hq_default_node(uint64_t N, uint32_t most) {
   if (N > most) return kHqRefNode;

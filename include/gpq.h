@@ -201,7 +201,9 @@ typedef struct gpq_phold_config {
                              * works a heap of nodes up to 1,024 items, the whole GPU (one
                              * cooperative launch) larger ones; 0 = the population rounded up
                              * to a power of two (at least 2,048), or the reference's 256 K
-                             * (HQ_NODE_SIZE, src/config.h:88) above 4 M items */
+                             * (HQ_NODE_SIZE, src/config.h:88) above 4 M items, or where the
+                             * root does not fit in memory (a handle for 2.6 M items takes 1.15 GB
+                             * with one root, 0.32 GB with 256 K nodes) */
   uint32_t laq_mode;        /* LAQ: 0 = sorted runs, children merged each window; 1 = unordered
                                arrays, each window's safe events selected and ranked; 2 = time
                                buckets of 8-byte keys per LP, each window's buckets ranked
